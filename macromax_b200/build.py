@@ -8,9 +8,11 @@ from __future__ import annotations
 
 import hashlib
 import os
+import re
 import shutil
 import subprocess
 import sys
+from concurrent.futures import ThreadPoolExecutor
 
 PKG = os.path.dirname(os.path.abspath(__file__))
 ROOT = os.path.dirname(PKG)
@@ -20,8 +22,10 @@ LIB_NAME = 'libmacromax_b200.so'
 LIB_PATH = os.path.join(PKG, LIB_NAME)
 STAMP = LIB_PATH + '.srchash'
 
-SOURCES = ['mmx_capi.cu']
-NVCC_FLAGS = ['-gencode', 'arch=compute_100a,code=sm_100a', '-lineinfo', '-O3', '-std=c++17', '-shared',
+OBJ_DIR = os.path.join(PKG, '_build')
+# compiled side by side and linked into one library; a translation unit whose sources did not change keeps its object
+SOURCES = ['mmx_capi.cu', 'mmx_gen.cu', 'mmx_gen_f64.cu']
+NVCC_FLAGS = ['-gencode', 'arch=compute_100a,code=sm_100a', '-lineinfo', '-O3', '-std=c++17',
               '-Xcompiler', '-fPIC', '-Xcompiler', '-O2']
 
 
@@ -51,12 +55,48 @@ def up_to_date() -> bool:
         return f.read().strip() == _source_hash()
 
 
+def _unit_hash(source: str) -> str:
+    """Of one translation unit: its source, the files of this tree that it includes, and the flags."""
+    seen, todo = set(), [os.path.join(CSRC, source)]
+    h = hashlib.sha256(' '.join(NVCC_FLAGS).encode())
+    while todo:
+        path = os.path.normpath(todo.pop())
+        if path in seen or not os.path.exists(path):
+            continue
+        seen.add(path)
+        with open(path, 'rb') as f:
+            text = f.read()
+        h.update(os.path.basename(path).encode() + text)
+        todo += sorted(os.path.join(os.path.dirname(path), m) for m in re.findall(r'#include "([^"]+)"', text.decode()))
+    return h.hexdigest()
+
+
+def _compile(source: str, force: bool, verbose: bool) -> str:
+    obj = os.path.join(OBJ_DIR, source + '.o')
+    stamp = obj + '.srchash'
+    digest = _unit_hash(source)
+    if not force and os.path.exists(obj) and os.path.exists(stamp):
+        with open(stamp) as f:
+            if f.read().strip() == digest:
+                return obj
+    cmd = [_nvcc(), *NVCC_FLAGS, '-I', INCLUDE, '-c', '-o', obj + '.tmp', os.path.join(CSRC, source)]
+    if verbose:
+        print(' '.join(cmd), flush=True)
+    subprocess.run(cmd, check=True)
+    os.replace(obj + '.tmp', obj)
+    with open(stamp, 'w') as f:
+        f.write(digest)
+    return obj
+
+
 def build(force: bool = False, verbose: bool = False) -> str:
     if not force and up_to_date():
         return LIB_PATH
-    srcs = [os.path.join(CSRC, s) for s in SOURCES]
+    os.makedirs(OBJ_DIR, exist_ok=True)
+    with ThreadPoolExecutor(max_workers=min(len(SOURCES), os.cpu_count() or 1)) as pool:
+        objs = list(pool.map(lambda src: _compile(src, force, verbose), SOURCES))
     tmp = LIB_PATH + '.tmp'
-    cmd = [_nvcc(), *NVCC_FLAGS, '-I', INCLUDE, '-o', tmp, *srcs]
+    cmd = [_nvcc(), *NVCC_FLAGS[:2], '-shared', '-o', tmp, *objs]
     if verbose:
         print(' '.join(cmd), flush=True)
     subprocess.run(cmd, check=True)

@@ -12,6 +12,7 @@
 #include <vector>
 
 #include "mmx_fast.cuh"
+#include "mmx_gen.h"
 #include "mmx_reg.cuh"
 #include "mmx_plane.cuh"
 #include "mmx_epro.cuh"
@@ -109,6 +110,7 @@ struct PassCfg {
   size_t rc_smem = 0;
   int tma = 0;        // 1: strided pass staged by bulk tensor copies (k_tma_pass) through `tmap`
   CUtensorMap tmap;   // 5-D map of the work buffer [B][C][outer][N][inner], box 16 x N x 1 x C x 1
+  GenTile gen, gen3;  // the pass for any length (gen3: with a 3x3 chi); threads == 0: none
 };
 
 bool reg_length(int n, int C) { return C == 3 ? (n == 64 || n == 128) : (n == 64 || n == 128 || n == 256 || n == 512); }
@@ -686,18 +688,39 @@ int fast_dispatch(const PassCfg& pc, const IterArgs<float>& a, int C, int chi_ki
   }
 }
 
+// The any-length pass of a configuration that has one for this chi
+template <class R>
+int launch_gen(const PassCfg& pc, IterArgs<R> a, int C, int chi_kind, int batch, cudaStream_t s) {
+  const bool m = chi_kind != MMX_CHI_SCALAR;
+  GenKind kind = GEN_STRIDED;
+  int dir = -1;
+  switch (pc.ops) {
+    case OP_FWD: break;
+    case OP_INV: dir = +1; break;
+    case OP_FWD | OP_G | OP_INV: kind = GEN_GREEN; break;
+    case OP_PRO | OP_FWD: kind = m ? GEN_PRO3 : GEN_PRO; break;
+    case OP_INV | OP_EPI: kind = m ? GEN_EPI3 : GEN_EPI; break;
+    default: return fail(MMX_ERR_ARG, "internal: operation set without an any-length kernel");
+  }
+  a.outer = pc.outer;
+  a.inner = pc.inner;
+  const GenTile& t = kind == GEN_PRO3 || kind == GEN_EPI3 ? pc.gen3 : pc.gen;
+  MMX_CUDA(gen_launch<R>(kind, t, a, C, chi_kind, dir, kind == GEN_STRIDED ? batch * C : batch, a.T, a.T, (R)1,
+                         pdl_enabled(), s));
+  return MMX_OK;
+}
+
 template <class R>
 int dispatch_pass(const PassCfg& pc, const IterArgs<R>& a, int C, int chi_kind, int batch, cudaStream_t s) {
+  if (C == 1 && chi_kind != MMX_CHI_SCALAR) return fail(MMX_ERR_ARG, "a 3x3 chi needs a 3-component field");
+  if (!pc.fast) {
+    const bool m = chi_kind != MMX_CHI_SCALAR && (pc.ops == (OP_PRO | OP_FWD) || pc.ops == (OP_INV | OP_EPI));
+    if ((m ? pc.gen3 : pc.gen).threads) return launch_gen<R>(pc, a, C, chi_kind, batch, s);
+  }
   if constexpr (std::is_same<R, float>::value) {
-    if (pc.fast) {
-      if (C == 1 && chi_kind != MMX_CHI_SCALAR) return fail(MMX_ERR_ARG, "a 3x3 chi needs a 3-component field");
-      return fast_dispatch(pc, a, C, chi_kind, batch, s);
-    }
+    if (pc.fast) return fast_dispatch(pc, a, C, chi_kind, batch, s);
   }
-  if (C == 1) {
-    if (chi_kind != MMX_CHI_SCALAR) return fail(MMX_ERR_ARG, "a 3x3 chi needs a 3-component field");
-    return dispatch_ops<R, 1, MMX_CHI_SCALAR>(pc, a, batch, s);
-  }
+  if (C == 1) return dispatch_ops<R, 1, MMX_CHI_SCALAR>(pc, a, batch, s);
   if (chi_kind == MMX_CHI_SCALAR) return dispatch_ops<R, 3, MMX_CHI_SCALAR>(pc, a, batch, s);
   if (chi_kind == MMX_CHI_SYM6) return dispatch_ops<R, 3, MMX_CHI_SYM6>(pc, a, batch, s);
   return dispatch_ops<R, 3, MMX_CHI_MAT3>(pc, a, batch, s);
@@ -819,6 +842,19 @@ std::vector<PassCfg> build_passes(const mmx_plan* p, bool defect) {
           pc.tiles = outer * inner / 8;
           pc.smem = ((size_t)tile_rows<8>(3 * n) * 8 + n) * sizeof(float2);
         }
+      }
+    }
+    if (ops_ok && !p->force_generic && (int64_t)p->batch * p->ncomp <= 65535) {
+      const bool dbl = p->prec == MMX_C128;
+      const int C = p->ncomp, sms = sm_count();
+      if (ops == (OP_PRO | OP_FWD) || ops == (OP_INV | OP_EPI)) {
+        const bool epi = (ops & OP_EPI) != 0;
+        pc.gen = gen_tile(epi ? GEN_EPI : GEN_PRO, n, C, dbl, outer, inner, p->batch, sms);
+        if (C == 3) pc.gen3 = gen_tile(epi ? GEN_EPI3 : GEN_PRO3, n, C, dbl, outer, inner, p->batch, sms);
+      } else if (ops & OP_G) {
+        pc.gen = gen_tile(GEN_GREEN, n, C, dbl, outer, inner, p->batch, sms);
+      } else {
+        pc.gen = gen_tile(GEN_STRIDED, n, 1, dbl, outer, inner, (int64_t)p->batch * C, sms);
       }
     }
     v.push_back(pc);
@@ -1053,6 +1089,20 @@ template <class R> int run_fftn(mmx_plan* p, const void* in, void* out, int64_t 
           cur_in = out;
           continue;
         }
+      }
+    }
+    if (!p->force_generic) {
+      const GenKind kind = inner > 1 ? GEN_STRIDED : GEN_ROWS;
+      const GenTile t = gen_tile(kind, p->ax[axis].n, 1, p->prec == MMX_C128, outer, inner, 1, sm_count());
+      const R sc = (R)((inverse && k == 0) ? 1.0 / (double)p->N : 1.0);
+      if (t.threads && (kind == GEN_ROWS || sc == (R)1)) {
+        IterArgs<R> a = base_args<R>(p);
+        a.ax = p->ax[axis];
+        a.outer = outer;
+        a.inner = inner;
+        MMX_CUDA(gen_launch<R>(kind, t, a, 1, MMX_CHI_SCALAR, inverse ? +1 : -1, 1, cur_in, out, sc, pdl_enabled(), s));
+        cur_in = out;
+        continue;
       }
     }
     PassCfg pc;

@@ -79,13 +79,13 @@ template <> __device__ __forceinline__ double2 to_prec<double>(double2 a) { retu
 #define MMX_C16_1 0.92387953251128675612818318939678828682  // cos(pi / 8)
 #define MMX_S16_1 0.38268343236508977172845998403039886676  // sin(pi / 8)
 
-template <class R, int DIR> __device__ __forceinline__ void bfly2(cpx<R>* u) {
+template <class R, int DIR> __host__ __device__ __forceinline__ void bfly2(cpx<R>* u) {
   cpx<R> a = u[0], b = u[1];
   u[0] = a + b;
   u[1] = a - b;
 }
 
-template <class R, int DIR> __device__ __forceinline__ void bfly4v(cpx<R>& a, cpx<R>& b, cpx<R>& c, cpx<R>& d) {
+template <class R, int DIR> __host__ __device__ __forceinline__ void bfly4v(cpx<R>& a, cpx<R>& b, cpx<R>& c, cpx<R>& d) {
   cpx<R> t0 = a + c, t1 = a - c, t2 = b + d, t3 = mul_i(b - d, DIR);
   a = t0 + t2;
   c = t0 - t2;
@@ -93,9 +93,9 @@ template <class R, int DIR> __device__ __forceinline__ void bfly4v(cpx<R>& a, cp
   d = t1 - t3;
 }
 
-template <class R, int DIR> __device__ __forceinline__ void bfly4(cpx<R>* u) { bfly4v<R, DIR>(u[0], u[1], u[2], u[3]); }
+template <class R, int DIR> __host__ __device__ __forceinline__ void bfly4(cpx<R>* u) { bfly4v<R, DIR>(u[0], u[1], u[2], u[3]); }
 
-template <class R, int DIR> __device__ __forceinline__ void bfly3(cpx<R>* u) {
+template <class R, int DIR> __host__ __device__ __forceinline__ void bfly3(cpx<R>* u) {
   cpx<R> a = u[0], b = u[1], c = u[2];
   cpx<R> t = b + c;
   cpx<R> m = a - (R)0.5 * t;
@@ -105,7 +105,7 @@ template <class R, int DIR> __device__ __forceinline__ void bfly3(cpx<R>* u) {
   u[2] = m - s;
 }
 
-template <class R, int DIR> __device__ __forceinline__ void bfly5(cpx<R>* u) {
+template <class R, int DIR> __host__ __device__ __forceinline__ void bfly5(cpx<R>* u) {
   cpx<R> a = u[0];
   cpx<R> t1 = u[1] + u[4], t2 = u[2] + u[3], t3 = u[1] - u[4], t4 = u[2] - u[3];
   cpx<R> m1 = a + (R)MMX_C5_1 * t1 + (R)MMX_C5_2 * t2;
@@ -120,16 +120,16 @@ template <class R, int DIR> __device__ __forceinline__ void bfly5(cpx<R>* u) {
 }
 
 // multiply by exp(DIR * 2 pi i / 8) (k = 1), exp(DIR * 2 pi i 2/8) = DIR*i (k = 2), exp(DIR * 2 pi i 3/8) (k = 3)
-template <class R, int DIR> __device__ __forceinline__ cpx<R> w8_1(cpx<R> a) {
+template <class R, int DIR> __host__ __device__ __forceinline__ cpx<R> w8_1(cpx<R> a) {
   // (1 + DIR i) / sqrt 2
   return mkc<R>((a.x - DIR * a.y) * (R)MMX_SQRT1_2, (a.y + DIR * a.x) * (R)MMX_SQRT1_2);
 }
-template <class R, int DIR> __device__ __forceinline__ cpx<R> w8_3(cpx<R> a) {
+template <class R, int DIR> __host__ __device__ __forceinline__ cpx<R> w8_3(cpx<R> a) {
   // (-1 + DIR i) / sqrt 2
   return mkc<R>((-a.x - DIR * a.y) * (R)MMX_SQRT1_2, (-a.y + DIR * a.x) * (R)MMX_SQRT1_2);
 }
 
-template <class R, int DIR> __device__ __forceinline__ void bfly8(cpx<R>* u) {
+template <class R, int DIR> __host__ __device__ __forceinline__ void bfly8(cpx<R>* u) {
   // even/odd split: E = DFT4(u0,u2,u4,u6), O = DFT4(u1,u3,u5,u7); X_k = E_k + w^k O_k, X_{k+4} = E_k - w^k O_k
   cpx<R> e0 = u[0], e1 = u[2], e2 = u[4], e3 = u[6];
   cpx<R> o0 = u[1], o1 = u[3], o2 = u[5], o3 = u[7];
@@ -148,7 +148,7 @@ template <class R, int DIR> __device__ __forceinline__ void bfly8(cpx<R>* u) {
   u[7] = e3 - o3;
 }
 
-template <class R, int DIR> __device__ __forceinline__ void bfly16(cpx<R>* u) {
+template <class R, int DIR> __host__ __device__ __forceinline__ void bfly16(cpx<R>* u) {
   // x[n1 + 4 n2]: DFT4 over n2 for each n1, twiddle w16^(n1 k2), DFT4 over n1; X[k2 + 4 k1]
   cpx<R> y[16];
 #pragma unroll
@@ -203,7 +203,7 @@ template <class R, int RAD, int DIR> __device__ __forceinline__ void bfly_direct
   }
 }
 
-template <class R, int RAD, int DIR> __device__ __forceinline__ void bfly(cpx<R>* u, const cpx<R>* tw, int n) {
+template <class R, int RAD, int DIR> __host__ __device__ __forceinline__ void bfly(cpx<R>* u, const cpx<R>* tw, int n) {
   if constexpr (RAD == 2) bfly2<R, DIR>(u);
   else if constexpr (RAD == 3) bfly3<R, DIR>(u);
   else if constexpr (RAD == 4) bfly4<R, DIR>(u);

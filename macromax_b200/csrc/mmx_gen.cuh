@@ -1,0 +1,492 @@
+// FFT passes of the iteration (and of mmx_fftn) for axes of any length with prime factors up to 13, complex64 and
+// complex128.
+//
+// Self-sorting stages as in mmx_fft.cuh, but with radices up to 16 (two stages up to 256 samples, three up to 4096), so
+// that a pass exchanges its samples through shared memory once or twice, and as in mmx_reg.cuh the first stage reads
+// global memory into registers and the last one writes it (or the epilogue's results) from registers.  The length is a
+// run-time value: a stage is a switch over the radix around a fully unrolled butterfly, and the only divisions left,
+// of a butterfly's index by the stage's span and of a flat index by the butterflies per pencil, are multiplications by
+// a reciprocal that the host computes.  Stages between two shared-memory buffers need one barrier each.  What bounds
+// the passes is the traffic between L2 and the SMs; the runtime-radix passes of mmx_kernels.cuh (staged through shared
+// memory at both ends, out-of-line stages at a 64-register budget, integer divisions per element, twiddles from
+// global memory and O(r^2) butterflies for 7, 11 and 13) took five to ten times as long.
+//
+// Strided tiles: P = 2^lP consecutive pencils, shared memory [component][sample][pencil]; a warp's accesses are whole
+// rows.  Contiguous tiles: P rows of every component, shared memory [row][sample] with a skew of one word per 128 bytes.
+#pragma once
+#include <type_traits>
+
+#include "mmx_dft.cuh"
+#include "mmx_gen.h"
+
+template <class R> struct GenArgs : IterArgs<R> {
+  GenAxis g;
+  int lP;
+  int C;
+  const cpx<R>* in;
+  cpx<R>* out;
+  R scale;
+};
+
+__device__ __forceinline__ unsigned gen_div(unsigned x, unsigned m) { return __umulhi(x, m); }
+
+template <class F> __device__ __forceinline__ void radix_switch(int r, F&& f) {
+  switch (r) {
+    case 2: f(std::integral_constant<int, 2>{}); break;
+    case 3: f(std::integral_constant<int, 3>{}); break;
+    case 4: f(std::integral_constant<int, 4>{}); break;
+    case 5: f(std::integral_constant<int, 5>{}); break;
+    case 6: f(std::integral_constant<int, 6>{}); break;
+    case 7: f(std::integral_constant<int, 7>{}); break;
+    case 8: f(std::integral_constant<int, 8>{}); break;
+    case 9: f(std::integral_constant<int, 9>{}); break;
+    case 10: f(std::integral_constant<int, 10>{}); break;
+    case 11: f(std::integral_constant<int, 11>{}); break;
+    case 12: f(std::integral_constant<int, 12>{}); break;
+    case 13: f(std::integral_constant<int, 13>{}); break;
+    case 14: f(std::integral_constant<int, 14>{}); break;
+    case 15: f(std::integral_constant<int, 15>{}); break;
+    default: f(std::integral_constant<int, 16>{}); break;
+  }
+}
+
+// Inputs ld(i + q T) of butterfly i, twiddled, and its DFT in u; returns the index of its first output (the others follow
+// at the span L).  FIRST: span 1, no twiddles.
+template <class R, int RAD, int DIR, bool FIRST, class Ld>
+__device__ __forceinline__ int gen_dft(int i, int T, int L, unsigned mL, const cpx<R>* tw, cpx<R>* u, Ld&& ld) {
+#pragma unroll
+  for (int q = 0; q < RAD; ++q) u[q] = ld(i + q * T);
+  int k = 0;
+  if constexpr (!FIRST) {
+    if (L > 1) {
+      k = i - (int)gen_div((unsigned)i, mL) * L;
+      const int step = k * (int)gen_div((unsigned)T, mL);  // k n / (L RAD)
+#pragma unroll
+      for (int q = 1; q < RAD; ++q) {
+        cpx<R> w = tw[q * step];
+        if (DIR > 0) w = conjc(w);
+        u[q] = u[q] * w;
+      }
+    }
+  }
+  gdft<R, RAD, DIR>(u);
+  return (i - k) * RAD + k;
+}
+template <class R, int RAD, int DIR, bool FIRST, class Ld, class St>
+__device__ __forceinline__ void gen_butterfly(int i, int T, int L, unsigned mL, const cpx<R>* tw, Ld&& ld, St&& st) {
+  cpx<R> u[RAD];
+  const int d0 = gen_dft<R, RAD, DIR, FIRST>(i, T, L, mL, tw, u, ld);
+  const int Ls = FIRST ? 1 : L;
+#pragma unroll
+  for (int q = 0; q < RAD; ++q) st(d0 + q * Ls, u[q]);
+}
+
+// -i alpha_i / (|k|^2 - alpha) / N (solver.py:566-568, with the 1/N of the inverse transform)
+template <class R> struct GenGreen {
+  R ar, ai, ai2, s;
+  __device__ __forceinline__ cpx<R> operator()(R k2) const {
+    const R dr = k2 - ar;
+    const R inv = s / (dr * dr + ai2);
+    return mkc<R>(ai2 * inv, -ai * dr * inv);
+  }
+};
+
+// registers: 85 (complex64) and 128 (complex128) per thread at 256 threads
+template <class R> struct GenBounds { static constexpr int min_blocks = sizeof(R) == 4 ? 3 : 2; };
+
+// ---------------------------------------------------------------------------------------------------------------
+// Strided axis, FFT only.  blockIdx.y: component plane (right-hand side * C + component), or transform.
+// ---------------------------------------------------------------------------------------------------------------
+template <class R, int DIR>
+__global__ void __launch_bounds__(256, GenBounds<R>::min_blocks) k_gen_strided(const __grid_constant__ GenArgs<R> a) {
+  extern __shared__ __align__(16) unsigned char mmx_smem_raw[];
+  const int n = a.g.n, lP = a.lP, P = 1 << lP, nst = a.g.nst;
+  cpx<R>* sm = reinterpret_cast<cpx<R>*>(mmx_smem_raw);
+  cpx<R>* tw = sm + ((size_t)n << lP) * (nst > 2 ? 2 : 1);
+  const cpx<R>* twg = (const cpx<R>*)a.ax.tw;
+  for (int t = threadIdx.x; t < n; t += blockDim.x) tw[t] = twg[t];  // published by the first stage's barrier
+  const int pl = threadIdx.x & (P - 1), slot = threadIdx.x >> lP, nslots = blockDim.x >> lP;
+  const unsigned inner = (unsigned)a.inner;
+  const int64_t p = (int64_t)blockIdx.x * P + pl;
+  const bool valid = p < a.outer * a.inner;
+  const int64_t o = p / inner;
+  const int64_t off = (int64_t)blockIdx.y * a.N + o * n * inner + (p - o * inner);
+  pdl_wait();
+  pdl_trigger();
+  if (a.st && !a.st[blockIdx.y / a.C].active) return;
+  const cpx<R>* gi = a.in + off;
+  cpx<R>* go = a.out + off;
+  radix_switch(a.g.r[0], [&](auto rad) {
+    constexpr int RAD = decltype(rad)::value;
+    const int T = a.g.T[0];
+    for (int i = slot; i < T; i += nslots)
+      gen_butterfly<R, RAD, DIR, true>(
+          i, T, 1, 0u, tw, [&](int j) { return valid ? gi[(unsigned)j * inner] : mkc<R>((R)0, (R)0); },
+          [&](int j, cpx<R> v) { sm[(j << lP) + pl] = v; });
+  });
+  __syncthreads();
+  cpx<R>* cur = sm;
+  for (int s = 1; s + 1 < nst; ++s) {
+    cpx<R>* dst = cur == sm ? sm + ((size_t)n << lP) : sm;
+    radix_switch(a.g.r[s], [&](auto rad) {
+      constexpr int RAD = decltype(rad)::value;
+      const int T = a.g.T[s];
+      for (int i = slot; i < T; i += nslots)
+        gen_butterfly<R, RAD, DIR, false>(
+            i, T, a.g.L[s], a.g.mL[s], tw, [&](int j) { return cur[(j << lP) + pl]; },
+            [&](int j, cpx<R> v) { dst[(j << lP) + pl] = v; });
+    });
+    __syncthreads();
+    cur = dst;
+  }
+  if (!valid) return;
+  radix_switch(a.g.r[nst - 1], [&](auto rad) {
+    constexpr int RAD = decltype(rad)::value;
+    const int T = a.g.T[nst - 1];
+    for (int i = slot; i < T; i += nslots)
+      gen_butterfly<R, RAD, DIR, false>(
+          i, T, T, a.g.mL[nst - 1], tw, [&](int j) { return cur[(j << lP) + pl]; },
+          [&](int j, cpx<R> v) { go[(unsigned)j * inner] = v; });
+  });
+}
+
+// ---------------------------------------------------------------------------------------------------------------
+// Axis 0: forward FFT, Green multiply, inverse FFT.  blockIdx.y: right-hand side.
+// ---------------------------------------------------------------------------------------------------------------
+template <class R, int C>
+__global__ void __launch_bounds__(256, GenBounds<R>::min_blocks) k_gen_green(const __grid_constant__ GenArgs<R> a) {
+  extern __shared__ __align__(16) unsigned char mmx_smem_raw[];
+  const int n = a.g.n, lP = a.lP, P = 1 << lP, nst = a.g.nst;
+  const size_t words = ((size_t)C * n) << lP;
+  cpx<R>* sm = reinterpret_cast<cpx<R>*>(mmx_smem_raw);
+  cpx<R>* tw = sm + 2 * words;
+  R* sk0 = reinterpret_cast<R*>(tw + n);
+  const cpx<R>* twg = (const cpx<R>*)a.ax.tw;
+  for (int t = threadIdx.x; t < n; t += blockDim.x) {
+    tw[t] = twg[t];
+    sk0[t] = a.kv[0][t];
+  }
+  const int b = blockIdx.y;
+  const mmx_rhs_state* st = a.st + b;
+  const int pl = threadIdx.x & (P - 1), slot = threadIdx.x >> lP, nslots = blockDim.x >> lP;
+  const unsigned inner = (unsigned)a.inner;  // axis 0 has outer == 1: a pencil is its inner index
+  const unsigned p = blockIdx.x * P + pl;
+  const bool valid = p < inner;
+  R k1 = (R)0, k2 = (R)0;
+  if (valid) {
+    if (a.ndim == 3) {
+      const unsigned i1 = p / (unsigned)a.dims[2];
+      k1 = a.kv[1][i1];
+      k2 = a.kv[2][p - i1 * (unsigned)a.dims[2]];
+    } else if (a.ndim == 2) {
+      k1 = a.kv[1][p];
+    }
+  }
+  pdl_wait();
+  pdl_trigger();
+  if (!st->active) return;
+  cpx<R>* g = a.T + (int64_t)b * C * a.N + p;
+  const R kt2 = k1 * k1 + k2 * k2;
+  const R ar = (R)st->alpha_re, ai = (R)st->alpha_im;
+  const GenGreen<R> green{ar, ai, ai * ai, a.inv_total};
+  auto component = [&](int& i, int T) {  // i in [0, C T) -> component, i mod T
+    int c = 0;
+    if constexpr (C == 3) {
+      c = (i >= T) + (i >= 2 * T);
+      i -= c * T;
+    }
+    return c;
+  };
+  radix_switch(a.g.r[0], [&](auto rad) {
+    constexpr int RAD = decltype(rad)::value;
+    const int T = a.g.T[0];
+    for (int e = slot; e < C * T; e += nslots) {
+      int i = e;
+      const int c = component(i, T);
+      const cpx<R>* gi = g + (int64_t)c * a.N;
+      cpx<R>* d = sm + (((size_t)c * n) << lP) + pl;
+      gen_butterfly<R, RAD, -1, true>(
+          i, T, 1, 0u, tw, [&](int j) { return valid ? gi[(unsigned)j * inner] : mkc<R>((R)0, (R)0); },
+          [&](int j, cpx<R> v) { d[j << lP] = v; });
+    }
+  });
+  __syncthreads();
+  cpx<R>*cur = sm, *oth = sm + words;
+  for (int s = 1; s < nst; ++s) {
+    const bool with_green = C == 1 && s + 1 == nst;
+    radix_switch(a.g.r[s], [&](auto rad) {
+      constexpr int RAD = decltype(rad)::value;
+      const int T = a.g.T[s];
+      for (int e = slot; e < C * T; e += nslots) {
+        int i = e;
+        const int c = component(i, T);
+        const size_t base = (((size_t)c * n) << lP) + pl;
+        gen_butterfly<R, RAD, -1, false>(
+            i, T, a.g.L[s], a.g.mL[s], tw, [&](int j) { return cur[base + (j << lP)]; },
+            [&](int j, cpx<R> v) {
+              if (with_green) v = v * green(sk0[j] * sk0[j] + kt2);
+              oth[base + (j << lP)] = v;
+            });
+      }
+    });
+    __syncthreads();
+    cpx<R>* t = cur;
+    cur = oth;
+    oth = t;
+  }
+  if constexpr (C == 3) {
+    // the dyadic split g (F - P_L F) + (i alpha_i / alpha) P_L F (solver.py:571-577, backend/__init__.py:606-649), with
+    // the reference's DC rule and no longitudinal part along absent axes
+    const cpx<R> h = divc(mkc<R>((R)0, ai), mkc<R>(ar, ai)) * a.inv_total;
+    for (int j = slot; j < n; j += nslots) {
+      const R k0 = sk0[j];
+      const R kk2 = k0 * k0 + kt2;
+      const cpx<R> gf = green(kk2);
+      const R kv[3] = {k0, k1, k2};
+      cpx<R> F[3], PL[3];
+#pragma unroll
+      for (int c = 0; c < 3; ++c) F[c] = cur[((size_t)(c * n + j) << lP) + pl];
+      if (j == 0 && p == 0) {
+#pragma unroll
+        for (int c = 0; c < 3; ++c) PL[c] = c < a.ndim ? F[c] : mkc<R>((R)0, (R)0);
+      } else {
+        cpx<R> proj = mkc<R>((R)0, (R)0);
+#pragma unroll
+        for (int c = 0; c < 3; ++c)
+          if (c < a.ndim) proj += kv[c] * F[c];
+        proj = proj * ((R)1 / kk2);
+#pragma unroll
+        for (int c = 0; c < 3; ++c) PL[c] = c < a.ndim ? kv[c] * proj : mkc<R>((R)0, (R)0);
+      }
+#pragma unroll
+      for (int c = 0; c < 3; ++c) cur[((size_t)(c * n + j) << lP) + pl] = gf * (F[c] - PL[c]) + h * PL[c];
+    }
+    __syncthreads();
+  }
+  for (int s = 0; s + 1 < nst; ++s) {
+    radix_switch(a.g.r[s], [&](auto rad) {
+      constexpr int RAD = decltype(rad)::value;
+      const int T = a.g.T[s];
+      for (int e = slot; e < C * T; e += nslots) {
+        int i = e;
+        const int c = component(i, T);
+        const size_t base = (((size_t)c * n) << lP) + pl;
+        gen_butterfly<R, RAD, +1, false>(
+            i, T, a.g.L[s], a.g.mL[s], tw, [&](int j) { return cur[base + (j << lP)]; },
+            [&](int j, cpx<R> v) { oth[base + (j << lP)] = v; });
+      }
+    });
+    __syncthreads();
+    cpx<R>* t = cur;
+    cur = oth;
+    oth = t;
+  }
+  if (!valid) return;
+  radix_switch(a.g.r[nst - 1], [&](auto rad) {
+    constexpr int RAD = decltype(rad)::value;
+    const int T = a.g.T[nst - 1];
+    for (int e = slot; e < C * T; e += nslots) {
+      int i = e;
+      const int c = component(i, T);
+      const size_t base = (((size_t)c * n) << lP) + pl;
+      cpx<R>* go = g + (int64_t)c * a.N;
+      gen_butterfly<R, RAD, +1, false>(
+          i, T, T, a.g.mL[nst - 1], tw, [&](int j) { return cur[base + (j << lP)]; },
+          [&](int j, cpx<R> v) { go[(unsigned)j * inner] = v; });
+    }
+  });
+}
+
+// ---------------------------------------------------------------------------------------------------------------
+// Contiguous axis.  A tile holds P rows of each of the C components: row r of the tile is component r >> lP, row
+// r & (P - 1) of the P rows.  KIND: GEN_ROWS (in -> out, C = 1), GEN_PRO, GEN_EPI, GEN_PRO3, GEN_EPI3.
+// ---------------------------------------------------------------------------------------------------------------
+template <class R> struct GenSkew { static constexpr int shift = sizeof(R) == 4 ? 4 : 3; };
+template <class R> __host__ __device__ __forceinline__ int gen_pitch(int n) { return n + (n >> GenSkew<R>::shift); }
+template <class R> __device__ __forceinline__ int gen_at(int j) { return j + (j >> GenSkew<R>::shift); }
+
+template <class R, int KIND, int CHI, int DIR>
+__global__ void __launch_bounds__(256, GenBounds<R>::min_blocks) k_gen_rows(const __grid_constant__ GenArgs<R> a) {
+  constexpr bool kPro = KIND == GEN_PRO, kEpi = KIND == GEN_EPI, kPro3 = KIND == GEN_PRO3, kEpi3 = KIND == GEN_EPI3;
+  extern __shared__ __align__(16) unsigned char mmx_smem_raw[];
+  const int n = a.g.n, lP = a.lP, P = 1 << lP, nst = a.g.nst;
+  const int C = KIND == GEN_ROWS ? 1 : (kPro3 || kEpi3) ? 3 : a.C;
+  const int rows = C << lP, pitch = gen_pitch<R>(n);
+  const int words = rows * pitch;
+  cpx<R>* sm = reinterpret_cast<cpx<R>*>(mmx_smem_raw);
+  cpx<R>* tw = sm + (size_t)words * ((nst > 2 || kPro3 || kEpi3) ? 2 : 1);
+  const cpx<R>* twg = (const cpx<R>*)a.ax.tw;
+  for (int t = threadIdx.x; t < n; t += blockDim.x) tw[t] = twg[t];
+  const int b = blockIdx.y;
+  const int64_t row0 = (int64_t)blockIdx.x << lP;
+  const int left = a.outer - row0 < P ? (int)(a.outer - row0) : P;  // rows of this tile within the field
+  const int64_t N = a.N;
+  pdl_wait();
+  pdl_trigger();
+  ChiCoef<R> cc;
+  const cpx<R>* Ecur = nullptr;
+  cpx<R>* Eoth = nullptr;
+  const mmx_rhs_state* st = a.st + b;
+  if constexpr (KIND != GEN_ROWS) {
+    if (!st->active) return;
+    cc = chi_coef<R>(st);
+    const int cur = st->cur;
+    const int64_t fbase = (int64_t)b * C * N + row0 * n;
+    Ecur = (cur ? a.E1 : a.E0) + fbase;
+    Eoth = (cur ? a.E0 : a.E1) + fbase;
+  }
+  // first word of tile row r relative to the tile's first word of component 0
+  auto row_off = [&](int r) { return (int64_t)(r >> lP) * N + (int64_t)(r & (P - 1)) * n; };
+  const cpx<R>* gi = KIND == GEN_ROWS ? a.in + row0 * n : a.T + (int64_t)b * C * N + row0 * n;
+  cpx<R>* go = KIND == GEN_ROWS ? a.out + row0 * n : a.T + (int64_t)b * C * N + row0 * n;
+  const cpx<R>* __restrict__ X = a.chi + row0 * n;
+  const cpx<R>* __restrict__ S = a.src + (int64_t)b * C * N + row0 * n;
+
+  cpx<R>* cur = sm;
+  int s0 = 0;  // the next stage
+  if constexpr (kPro3) {
+    // all components of a voxel in one thread, chi E + s' to shared memory
+#pragma unroll 2
+    for (int e = threadIdx.x; e < left * n; e += blockDim.x) {
+      const int row = (int)gen_div((unsigned)e, a.g.mn), j = e - row * n;
+      cpx<R> v[3], t[3];
+#pragma unroll
+      for (int c = 0; c < 3; ++c) v[c] = Ecur[c * N + e];
+      apply_chi<R, 3, CHI>(X, N, e, cc, v, t);
+#pragma unroll
+      for (int c = 0; c < 3; ++c) {
+        if (!source_is_zero(st, c)) t[c] += cc.s * S[c * N + e];
+        sm[((c << lP) + row) * pitch + gen_at<R>(j)] = t[c];
+      }
+    }
+    __syncthreads();
+  } else {
+    radix_switch(a.g.r[0], [&](auto rad) {
+      constexpr int RAD = decltype(rad)::value;
+      const int T = a.g.T[0];
+      for (int e = threadIdx.x; e < rows * T; e += blockDim.x) {
+        const int r = (int)gen_div((unsigned)e, a.g.mT[0]), i = e - r * T;
+        if ((r & (P - 1)) >= left) continue;
+        const int64_t off = row_off(r);
+        cpx<R>* d = sm + r * pitch;
+        if constexpr (kPro) {
+          const cpx<R>*eS = Ecur + off, *sS = S + off, *xS = X + (int64_t)(r & (P - 1)) * n;
+          const bool with_src = !source_is_zero(st, r >> lP);
+          gen_butterfly<R, RAD, DIR, true>(
+              i, T, 1, 0u, tw,
+              [&](int j) {
+                cpx<R> v = (cc.a * xS[j] + cc.b) * eS[j];
+                if (with_src) v += cc.s * sS[j];
+                return v;
+              },
+              [&](int j, cpx<R> v) { d[gen_at<R>(j)] = v; });
+        } else {
+          const cpx<R>* tS = gi + off;
+          gen_butterfly<R, RAD, DIR, true>(
+              i, T, 1, 0u, tw, [&](int j) { return KIND == GEN_ROWS ? tS[j] * a.scale : tS[j]; },
+              [&](int j, cpx<R> v) { d[gen_at<R>(j)] = v; });
+        }
+      }
+    });
+    __syncthreads();
+    s0 = 1;
+  }
+  const int s1 = kEpi3 ? nst : nst - 1;  // the stages between shared-memory buffers
+  for (int s = s0; s < s1; ++s) {
+    cpx<R>* dst = cur == sm ? sm + words : sm;
+    radix_switch(a.g.r[s], [&](auto rad) {
+      constexpr int RAD = decltype(rad)::value;
+      const int T = a.g.T[s];
+      for (int e = threadIdx.x; e < rows * T; e += blockDim.x) {
+        const int r = (int)gen_div((unsigned)e, a.g.mT[s]), i = e - r * T;
+        const cpx<R>* src = cur + r * pitch;
+        cpx<R>* d = dst + r * pitch;
+        gen_butterfly<R, RAD, DIR, false>(
+            i, T, a.g.L[s], a.g.mL[s], tw, [&](int j) { return src[gen_at<R>(j)]; },
+            [&](int j, cpx<R> v) { d[gen_at<R>(j)] = v; });
+      }
+    });
+    __syncthreads();
+    cur = dst;
+  }
+  double dd2 = 0.0, en2 = 0.0;
+  if constexpr (kEpi3) {
+    // V voxels per thread and round, all their loads ahead of their stores
+    constexpr int V = sizeof(R) == 4 ? 2 : 1;
+    const int count = left * n;
+    for (int e0 = threadIdx.x; e0 < count; e0 += V * blockDim.x) {
+      cpx<R> ev[V][3], d[V][3];
+#pragma unroll
+      for (int v = 0; v < V; ++v) {
+        const int e = e0 + v * blockDim.x;
+        if (e < count) {
+          const int row = (int)gen_div((unsigned)e, a.g.mn), j = e - row * n;
+          cpx<R> t[3];
+#pragma unroll
+          for (int c = 0; c < 3; ++c) {
+            ev[v][c] = Ecur[c * N + e];
+            t[c] = cur[((c << lP) + row) * pitch + gen_at<R>(j)] - ev[v][c];
+          }
+          apply_chi<R, 3, CHI>(X, N, e, cc, t, d[v]);
+        }
+      }
+#pragma unroll
+      for (int v = 0; v < V; ++v) {
+        const int e = e0 + v * blockDim.x;
+        if (e < count) {
+#pragma unroll
+          for (int c = 0; c < 3; ++c) {
+            const cpx<R> en = ev[v][c] + d[v][c];
+            Eoth[c * N + e] = en;
+            dd2 += norm2d(d[v][c]);
+            en2 += norm2d(en);
+          }
+        }
+      }
+    }
+  } else {
+    radix_switch(a.g.r[nst - 1], [&](auto rad) {
+      constexpr int RAD = decltype(rad)::value;
+      const int T = a.g.T[nst - 1];
+      for (int e = threadIdx.x; e < rows * T; e += blockDim.x) {
+        const int r = (int)gen_div((unsigned)e, a.g.mT[nst - 1]), i = e - r * T;
+        if ((r & (P - 1)) >= left) continue;
+        const int64_t off = row_off(r);
+        const cpx<R>* src = cur + r * pitch;
+        if constexpr (kEpi) {
+          const cpx<R>*eS = Ecur + off, *xS = X + (int64_t)(r & (P - 1)) * n;
+          cpx<R>* eO = Eoth + off;
+          cpx<R> u[RAD];
+          gen_dft<R, RAD, DIR, false>(i, T, T, a.g.mL[nst - 1], tw, u, [&](int j) { return src[gen_at<R>(j)]; });
+          // the outputs at i + q T: E and chi of CH of them are in flight at a time
+          constexpr int CH = RAD <= 8 ? RAD : (RAD + 1) / 2;
+#pragma unroll
+          for (int q0 = 0; q0 < RAD; q0 += CH) {
+            cpx<R> ev[CH], xv[CH];
+#pragma unroll
+            for (int q = 0; q < CH; ++q)
+              if (q0 + q < RAD) {
+                ev[q] = eS[i + (q0 + q) * T];
+                xv[q] = xS[i + (q0 + q) * T];
+              }
+#pragma unroll
+            for (int q = 0; q < CH; ++q)
+              if (q0 + q < RAD) {
+                const cpx<R> d = (cc.a * xv[q] + cc.b) * (u[q0 + q] - ev[q]);
+                const cpx<R> en = ev[q] + d;
+                eO[i + (q0 + q) * T] = en;
+                dd2 += norm2d(d);
+                en2 += norm2d(en);
+              }
+          }
+        } else {
+          cpx<R>* tO = go + off;
+          gen_butterfly<R, RAD, DIR, false>(
+              i, T, T, a.g.mL[nst - 1], tw, [&](int j) { return src[gen_at<R>(j)]; },
+              [&](int j, cpx<R> v) { tO[j] = v; });
+        }
+      }
+    });
+  }
+  if constexpr (kEpi || kEpi3) finish_pass_norms(a, b, dd2, en2);
+}
