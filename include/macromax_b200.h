@@ -191,6 +191,7 @@ int mmx_pointwise_mul(const void* A, int ra, int ca, const void* B, int cb, int 
 #define MMX_VARIANT_PLANE 8u          /* 3D, 128 x 128 planes, isotropic chi: the two inner axes in one pass */
 #define MMX_VARIANT_FUSED_EPILOGUE 16u /* epilogue fused with the next prologue (speculative); isotropic chi, and a 3x3 chi on 192-sample rows */
 #define MMX_VARIANT_TMA 32u            /* strided 128-sample passes staged by bulk tensor (TMA) copies */
+#define MMX_VARIANT_RUNTIME_RADIX 64u  /* the runtime-radix passes for lengths without a specialised kernel */
 
 /* Select the kernel variant of a plan (rebuilds its pass list, drops its captured graphs).  No reference
  * counterpart: the reference has one implementation per backend. */

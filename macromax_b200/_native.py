@@ -35,6 +35,7 @@ MMX_VARIANT_PERSISTENT = 4
 MMX_VARIANT_PLANE = 8
 MMX_VARIANT_FUSED_EPILOGUE = 16
 MMX_VARIANT_TMA = 32
+MMX_VARIANT_RUNTIME_RADIX = 64
 
 # numpy mirror of struct mmx_rhs_state (include/macromax_b200.h)
 STATE_DTYPE = np.dtype([

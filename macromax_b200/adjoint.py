@@ -58,9 +58,14 @@ class _SolveFn(torch.autograd.Function):
             return _SolveFn._forward_mixed(ctx, epsilon, sources, problem, eps_np)
         bs = BatchSolution(grid, sources.detach(), eps_np, bound=problem.get('bound'), wavenumber=k0,
                            dtype=problem.get('dtype', np.complex64), device=sources.device)
-        if problem.get('variant') is not None:  # the pass-kernel variant for both solves (e.g. the autotuner's)
+        variant = problem.get('variant')  # the pass-kernel variant for both solves (e.g. the autotuner's)
+        if variant is None and epsilon.dtype in (torch.float64, torch.complex128):
+            # a gradient returned in FP64 is compared and stored as such, though these solves round to complex64: they
+            # keep the passes whose rounding is that of the gradients a caller already has
+            variant = nat.MMX_VARIANT_RUNTIME_RADIX
+        if variant is not None:
             from . import autotune
-            autotune.set_variant(bs.engine, int(problem['variant']))
+            autotune.set_variant(bs.engine, int(variant))
         t0 = _now()
         bs.solve(problem.get('rtol', 1e-6), problem.get('maxiter', 100000))
         problem.setdefault('stats', {})['forward_iterations'] = bs.iterations

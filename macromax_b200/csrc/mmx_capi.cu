@@ -133,6 +133,7 @@ struct mmx_plan {
   FFTAxis ax[3];           // radix plans; tw points at device twiddles of the plan precision
   void* tw_dev[3] = {nullptr, nullptr, nullptr};
   void* kv_dev = nullptr;  // k tables, plan precision, concatenated
+  double* kvd_dev = nullptr;  // the same in FP64 (complex64 plans; complex128 plans use kv_dev)
   int kv_off[3] = {0, 0, 0};
   bool kv_set = false;
   void* work = nullptr;    // T [batch][ncomp][N]
@@ -151,6 +152,7 @@ struct mmx_plan {
   std::vector<PassCfg> plane_passes;  // the 3-pass schedule used when `plane` is set and chi is isotropic
   bool epro = false;           // fuse each epilogue with the next iteration's prologue
   bool tma = false;            // strided 128-sample passes staged by bulk tensor copies (k_tma_pass)
+  bool runtime_radix = false;  // k_iter_pass instead of the any-length passes (MMX_VARIANT_RUNTIME_RADIX)
   bool wide_green = false;     // MMX_WIDE_GREEN=1: 16-pencil tiles for the vector axis-0 pass (tests)
   std::vector<PassCfg> epro_passes;   // [middle passes..., EPI+PRO, repair]; the first PRO runs once per call
   // The last iteration call on this plan whose fused epilogue left the next iteration's first pass (the prologue
@@ -201,6 +203,7 @@ namespace {
 bool factorize(int n, FFTAxis& ax) {
   ax.n = n;
   ax.nst = 0;
+  ax.tw = ax.tw_lo = nullptr;
   int m = n;
   const int pref[] = {8, 4, 2, 3, 5, 7, 11, 13};
   while (m > 1) {
@@ -844,7 +847,7 @@ std::vector<PassCfg> build_passes(const mmx_plan* p, bool defect) {
         }
       }
     }
-    if (ops_ok && !p->force_generic && (int64_t)p->batch * p->ncomp <= 65535) {
+    if (ops_ok && !p->force_generic && !p->runtime_radix && (int64_t)p->batch * p->ncomp <= 65535) {
       const bool dbl = p->prec == MMX_C128;
       const int C = p->ncomp, sms = sm_count();
       if (ops == (OP_PRO | OP_FWD) || ops == (OP_INV | OP_EPI)) {
@@ -938,6 +941,8 @@ template <class R> IterArgs<R> base_args(mmx_plan* p) {
   for (int i = 0; i < 3; ++i) {
     a.dims[i] = (int)p->shape[i];
     a.kv[i] = p->kv_dev ? (const R*)p->kv_dev + p->kv_off[i] : nullptr;
+    const double* kd = p->prec == MMX_C128 ? (const double*)p->kv_dev : p->kvd_dev;
+    a.kvd[i] = kd ? kd + p->kv_off[i] : nullptr;
   }
   a.T = (cpx<R>*)p->work;
   a.partials = p->partials;
@@ -1100,7 +1105,8 @@ template <class R> int run_fftn(mmx_plan* p, const void* in, void* out, int64_t 
         a.ax = p->ax[axis];
         a.outer = outer;
         a.inner = inner;
-        MMX_CUDA(gen_launch<R>(kind, t, a, 1, MMX_CHI_SCALAR, inverse ? +1 : -1, 1, cur_in, out, sc, pdl_enabled(), s));
+        MMX_CUDA(gen_launch<R>(kind, t, a, 1, MMX_CHI_SCALAR, inverse ? +1 : -1, 1, cur_in, out, sc,
+                               pdl_enabled() && p->work, s));  // no plan: its twiddles are written on the stream
         cur_in = out;
         continue;
       }
@@ -1186,7 +1192,8 @@ int mmx_plan_create(int ndim, const int64_t* shape, int ncomp, int batch, int pr
       twd[2 * t] = std::cos(ang);
       twd[2 * t + 1] = std::sin(ang);
     }
-    cudaError_t e = cudaMalloc(&p->tw_dev[i], wb * n);
+    // complex64: the table, and behind it what rounding to float took from it
+    cudaError_t e = cudaMalloc(&p->tw_dev[i], (precision == MMX_C64 ? 2 : 1) * wb * n);
     if (e != cudaSuccess) {
       mmx_plan_destroy(p);
       return cuda_fail(e, "cudaMalloc(twiddles)");
@@ -1194,9 +1201,13 @@ int mmx_plan_create(int ndim, const int64_t* shape, int ncomp, int batch, int pr
     if (precision == MMX_C128) {
       e = cudaMemcpy(p->tw_dev[i], twd.data(), wb * n, cudaMemcpyHostToDevice);
     } else {
-      std::vector<float> twf(2 * (size_t)n);
-      for (size_t k = 0; k < twf.size(); ++k) twf[k] = (float)twd[k];
-      e = cudaMemcpy(p->tw_dev[i], twf.data(), wb * n, cudaMemcpyHostToDevice);
+      std::vector<float> twf(4 * (size_t)n);
+      for (size_t k = 0; k < twd.size(); ++k) {
+        twf[k] = (float)twd[k];
+        twf[twd.size() + k] = (float)(twd[k] - (double)twf[k]);
+      }
+      e = cudaMemcpy(p->tw_dev[i], twf.data(), 2 * wb * n, cudaMemcpyHostToDevice);
+      p->ax[i].tw_lo = (const float2*)p->tw_dev[i] + n;
     }
     if (e != cudaSuccess) {
       mmx_plan_destroy(p);
@@ -1208,6 +1219,7 @@ int mmx_plan_create(int ndim, const int64_t* shape, int ncomp, int batch, int pr
   }
   cudaError_t e = cudaMalloc(&p->kv_dev, (wb / 2) * (size_t)kv_total);
   if (e == cudaSuccess) e = cudaMemset(p->kv_dev, 0, (wb / 2) * (size_t)kv_total);
+  if (e == cudaSuccess && precision == MMX_C64) e = cudaMalloc(&p->kvd_dev, sizeof(double) * (size_t)kv_total);
   if (e == cudaSuccess) e = cudaMalloc(&p->work, wb * (size_t)batch * ncomp * p->N);
   if (e != cudaSuccess) {
     mmx_plan_destroy(p);
@@ -1271,6 +1283,7 @@ int mmx_plan_destroy(mmx_plan* p) {
   for (int i = 0; i < 3; ++i)
     if (p->tw_dev[i]) cudaFree(p->tw_dev[i]);
   if (p->kv_dev) cudaFree(p->kv_dev);
+  if (p->kvd_dev) cudaFree(p->kvd_dev);
   if (p->work) cudaFree(p->work);
   if (p->partials) cudaFree(p->partials);
   if (p->done) cudaFree(p->done);
@@ -1293,6 +1306,7 @@ int mmx_plan_set_kvectors(mmx_plan* p, const double* k) {
     std::vector<float> kf(total);
     for (int i = 0; i < total; ++i) kf[i] = (float)k[i];
     MMX_CUDA(cudaMemcpy(p->kv_dev, kf.data(), sizeof(float) * total, cudaMemcpyHostToDevice));
+    MMX_CUDA(cudaMemcpy(p->kvd_dev, k, sizeof(double) * total, cudaMemcpyHostToDevice));
   }
   p->kv_set = true;
   return MMX_OK;
@@ -1534,7 +1548,7 @@ extern "C" int mmx_iterate_graph_continue(mmx_plan* p, void* E0, void* E1, const
 
 extern "C" int mmx_plan_set_variant(mmx_plan* p, unsigned flags) {
   if (!p) return fail(MMX_ERR_ARG, "NULL plan");
-  if (flags & ~63u) return fail(MMX_ERR_ARG, "unknown variant flags");
+  if (flags & ~127u) return fail(MMX_ERR_ARG, "unknown variant flags");
   drop_graphs_of(p);  // captured graphs hold the previous kernels
   p->cont_valid = false;
   p->force_generic = (flags & MMX_VARIANT_GENERIC) != 0;
@@ -1543,6 +1557,7 @@ extern "C" int mmx_plan_set_variant(mmx_plan* p, unsigned flags) {
   p->plane = (flags & MMX_VARIANT_PLANE) != 0;
   p->epro = (flags & MMX_VARIANT_FUSED_EPILOGUE) != 0;
   p->tma = (flags & MMX_VARIANT_TMA) != 0;
+  p->runtime_radix = (flags & MMX_VARIANT_RUNTIME_RADIX) != 0;
   p->iter_passes = build_passes(p, false);
   p->defect_passes = build_passes(p, true);
   p->plane_passes = build_plane_passes(p);
@@ -1557,7 +1572,8 @@ extern "C" unsigned mmx_plan_get_variant(const mmx_plan* p) {
   if (!p) return 0u;
   return (p->force_generic ? MMX_VARIANT_GENERIC : 0u) | (p->no_reg ? MMX_VARIANT_SHARED_STAGED : 0u) |
          (p->pipe ? MMX_VARIANT_PERSISTENT : 0u) | (p->plane ? MMX_VARIANT_PLANE : 0u) |
-         (p->epro ? MMX_VARIANT_FUSED_EPILOGUE : 0u) | (p->tma ? MMX_VARIANT_TMA : 0u);
+         (p->epro ? MMX_VARIANT_FUSED_EPILOGUE : 0u) | (p->tma ? MMX_VARIANT_TMA : 0u) |
+         (p->runtime_radix ? MMX_VARIANT_RUNTIME_RADIX : 0u);
 }
 
 extern "C" int mmx_mat3_extremes(mmx_plan* p, const void* M, int64_t nvox, int mode, double ab, double* out_dev,

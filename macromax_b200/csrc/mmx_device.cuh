@@ -23,6 +23,7 @@ template <class R> struct IterArgs {
   int ndim;
   int dims[3];
   const R* kv[3];        // k-vector tables per axis
+  const double* kvd[3];  // the same in FP64
   cpx<R>* T;             // work [B][C][N]
   cpx<R>* E0;            // field buffers [B][C][N] (E0 is x for the defect)
   cpx<R>* E1;

@@ -24,6 +24,7 @@ struct FFTAxis {
   int nst;                    // number of stages
   int radix[MMX_MAX_STAGES];  // radices, product == n
   const void* tw;             // twiddle table cpx<R>[n]: exp(-2 pi i t / n)
+  const void* tw_lo;          // complex64: what rounding to float took from them, float2[n] (or null)
 };
 
 template <class R, int RAD, int DIR>

@@ -64,11 +64,12 @@ bool is_rows(GenKind k) { return k != GEN_STRIDED && k != GEN_GREEN; }
 size_t tile_bytes(GenKind kind, const GenAxis& ax, int C, int P, bool dbl) {
   const size_t wb = dbl ? 16 : 8;
   const size_t n = ax.n;
-  if (kind == GEN_STRIDED) return (n * P * (ax.nst > 2 ? 2 : 1) + n) * wb;
-  if (kind == GEN_GREEN) return (2 * C * n * P + n) * wb + n * wb / 2;
+  const size_t tables = n * 16;  // the twiddles: two floats or a double per part
+  if (kind == GEN_STRIDED) return n * P * (ax.nst > 2 ? 2 : 1) * wb + tables;
+  if (kind == GEN_GREEN) return 2 * C * n * P * wb + tables + n * sizeof(double);
   const size_t pitch = n + (n >> (dbl ? 3 : 4));
   const bool two = ax.nst > 2 || kind == GEN_PRO3 || kind == GEN_EPI3;
-  return (C * P * pitch * (two ? 2 : 1) + n) * wb;
+  return C * P * pitch * (two ? 2 : 1) * wb + tables;
 }
 
 }  // namespace

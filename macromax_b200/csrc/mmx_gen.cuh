@@ -28,6 +28,35 @@ template <class R> struct GenArgs : IterArgs<R> {
   R scale;
 };
 
+// A twiddle factor in shared memory: in complex64 as the sum of two floats, for the same reason as the coefficients of
+// mmx_dft.cuh (a length without tw_lo takes it as 0).
+template <class R> struct GenTw;
+template <> struct GenTw<float> {
+  using type = float4;
+  static __device__ __forceinline__ float4 load(const FFTAxis& ax, int t) {
+    const float2 h = ((const float2*)ax.tw)[t];
+    const float2 l = ax.tw_lo ? ((const float2*)ax.tw_lo)[t] : make_float2(0.f, 0.f);
+    return make_float4(h.x, h.y, l.x, l.y);
+  }
+  // u w (DIR < 0) or u conj(w)
+  template <int DIR> static __device__ __forceinline__ float2 mul(float2 u, float4 w) {
+    if (DIR > 0) {
+      w.y = -w.y;
+      w.w = -w.w;
+    }
+    return make_float2(fmaf(u.x, w.x, fmaf(-u.y, w.y, fmaf(u.x, w.z, -u.y * w.w))),
+                       fmaf(u.x, w.y, fmaf(u.y, w.x, fmaf(u.x, w.w, u.y * w.z))));
+  }
+};
+template <> struct GenTw<double> {
+  using type = double2;
+  static __device__ __forceinline__ double2 load(const FFTAxis& ax, int t) { return ((const double2*)ax.tw)[t]; }
+  template <int DIR> static __device__ __forceinline__ double2 mul(double2 u, double2 w) {
+    return DIR > 0 ? u * conjc(w) : u * w;
+  }
+};
+template <class R> using gtw = typename GenTw<R>::type;
+
 __device__ __forceinline__ unsigned gen_div(unsigned x, unsigned m) { return __umulhi(x, m); }
 
 template <class F> __device__ __forceinline__ void radix_switch(int r, F&& f) {
@@ -53,7 +82,7 @@ template <class F> __device__ __forceinline__ void radix_switch(int r, F&& f) {
 // Inputs ld(i + q T) of butterfly i, twiddled, and its DFT in u; returns the index of its first output (the others follow
 // at the span L).  FIRST: span 1, no twiddles.
 template <class R, int RAD, int DIR, bool FIRST, class Ld>
-__device__ __forceinline__ int gen_dft(int i, int T, int L, unsigned mL, const cpx<R>* tw, cpx<R>* u, Ld&& ld) {
+__device__ __forceinline__ int gen_dft(int i, int T, int L, unsigned mL, const gtw<R>* tw, cpx<R>* u, Ld&& ld) {
 #pragma unroll
   for (int q = 0; q < RAD; ++q) u[q] = ld(i + q * T);
   int k = 0;
@@ -62,18 +91,14 @@ __device__ __forceinline__ int gen_dft(int i, int T, int L, unsigned mL, const c
       k = i - (int)gen_div((unsigned)i, mL) * L;
       const int step = k * (int)gen_div((unsigned)T, mL);  // k n / (L RAD)
 #pragma unroll
-      for (int q = 1; q < RAD; ++q) {
-        cpx<R> w = tw[q * step];
-        if (DIR > 0) w = conjc(w);
-        u[q] = u[q] * w;
-      }
+      for (int q = 1; q < RAD; ++q) u[q] = GenTw<R>::template mul<DIR>(u[q], tw[q * step]);
     }
   }
   gdft<R, RAD, DIR>(u);
   return (i - k) * RAD + k;
 }
 template <class R, int RAD, int DIR, bool FIRST, class Ld, class St>
-__device__ __forceinline__ void gen_butterfly(int i, int T, int L, unsigned mL, const cpx<R>* tw, Ld&& ld, St&& st) {
+__device__ __forceinline__ void gen_butterfly(int i, int T, int L, unsigned mL, const gtw<R>* tw, Ld&& ld, St&& st) {
   cpx<R> u[RAD];
   const int d0 = gen_dft<R, RAD, DIR, FIRST>(i, T, L, mL, tw, u, ld);
   const int Ls = FIRST ? 1 : L;
@@ -81,13 +106,23 @@ __device__ __forceinline__ void gen_butterfly(int i, int T, int L, unsigned mL, 
   for (int q = 0; q < RAD; ++q) st(d0 + q * Ls, u[q]);
 }
 
-// -i alpha_i / (|k|^2 - alpha) / N (solver.py:566-568, with the 1/N of the inverse transform)
+// -i alpha_i / (|k|^2 - alpha) / N (solver.py:566-568, with the 1/N of the inverse transform), in FP64 and rounded once
+// (the field converges to the fixed point of the rounded g): complex64 starts the reciprocal in float and takes one
+// Newton step, about ten FP64 operations per sample.
 template <class R> struct GenGreen {
-  R ar, ai, ai2, s;
-  __device__ __forceinline__ cpx<R> operator()(R k2) const {
-    const R dr = k2 - ar;
-    const R inv = s / (dr * dr + ai2);
-    return mkc<R>(ai2 * inv, -ai * dr * inv);
+  double ar, ai, ai2, s;
+  __device__ __forceinline__ cpx<R> operator()(double k2) const {
+    const double dr = k2 - ar;
+    const double den = fma(dr, dr, ai2);
+    double r;
+    if constexpr (sizeof(R) == 4) {
+      r = (double)(1.0f / (float)den);
+      r = fma(r, fma(-den, r, 1.0), r);
+    } else {
+      r = 1.0 / den;
+    }
+    r *= s;
+    return mkc<R>((R)(ai2 * r), (R)(-ai * dr * r));
   }
 };
 
@@ -101,10 +136,10 @@ template <class R, int DIR>
 __global__ void __launch_bounds__(256, GenBounds<R>::min_blocks) k_gen_strided(const __grid_constant__ GenArgs<R> a) {
   extern __shared__ __align__(16) unsigned char mmx_smem_raw[];
   const int n = a.g.n, lP = a.lP, P = 1 << lP, nst = a.g.nst;
-  cpx<R>* sm = reinterpret_cast<cpx<R>*>(mmx_smem_raw);
-  cpx<R>* tw = sm + ((size_t)n << lP) * (nst > 2 ? 2 : 1);
-  const cpx<R>* twg = (const cpx<R>*)a.ax.tw;
-  for (int t = threadIdx.x; t < n; t += blockDim.x) tw[t] = twg[t];  // published by the first stage's barrier
+  gtw<R>* tw = reinterpret_cast<gtw<R>*>(mmx_smem_raw);
+  cpx<R>* sm = reinterpret_cast<cpx<R>*>(tw + n);
+  for (int t = threadIdx.x; t < n; t += blockDim.x)
+    tw[t] = GenTw<R>::load(a.ax, t);  // published by the first stage's barrier
   const int pl = threadIdx.x & (P - 1), slot = threadIdx.x >> lP, nslots = blockDim.x >> lP;
   const unsigned inner = (unsigned)a.inner;
   const int64_t p = (int64_t)blockIdx.x * P + pl;
@@ -158,13 +193,12 @@ __global__ void __launch_bounds__(256, GenBounds<R>::min_blocks) k_gen_green(con
   extern __shared__ __align__(16) unsigned char mmx_smem_raw[];
   const int n = a.g.n, lP = a.lP, P = 1 << lP, nst = a.g.nst;
   const size_t words = ((size_t)C * n) << lP;
-  cpx<R>* sm = reinterpret_cast<cpx<R>*>(mmx_smem_raw);
-  cpx<R>* tw = sm + 2 * words;
-  R* sk0 = reinterpret_cast<R*>(tw + n);
-  const cpx<R>* twg = (const cpx<R>*)a.ax.tw;
+  gtw<R>* tw = reinterpret_cast<gtw<R>*>(mmx_smem_raw);
+  cpx<R>* sm = reinterpret_cast<cpx<R>*>(tw + n);
+  double* sk0 = reinterpret_cast<double*>(sm + 2 * words);  // k of axis 0
   for (int t = threadIdx.x; t < n; t += blockDim.x) {
-    tw[t] = twg[t];
-    sk0[t] = a.kv[0][t];
+    tw[t] = GenTw<R>::load(a.ax, t);
+    sk0[t] = a.kvd[0][t];
   }
   const int b = blockIdx.y;
   const mmx_rhs_state* st = a.st + b;
@@ -172,23 +206,23 @@ __global__ void __launch_bounds__(256, GenBounds<R>::min_blocks) k_gen_green(con
   const unsigned inner = (unsigned)a.inner;  // axis 0 has outer == 1: a pencil is its inner index
   const unsigned p = blockIdx.x * P + pl;
   const bool valid = p < inner;
-  R k1 = (R)0, k2 = (R)0;
+  double k1 = 0.0, k2 = 0.0;
   if (valid) {
     if (a.ndim == 3) {
       const unsigned i1 = p / (unsigned)a.dims[2];
-      k1 = a.kv[1][i1];
-      k2 = a.kv[2][p - i1 * (unsigned)a.dims[2]];
+      k1 = a.kvd[1][i1];
+      k2 = a.kvd[2][p - i1 * (unsigned)a.dims[2]];
     } else if (a.ndim == 2) {
-      k1 = a.kv[1][p];
+      k1 = a.kvd[1][p];
     }
   }
   pdl_wait();
   pdl_trigger();
   if (!st->active) return;
   cpx<R>* g = a.T + (int64_t)b * C * a.N + p;
-  const R kt2 = k1 * k1 + k2 * k2;
-  const R ar = (R)st->alpha_re, ai = (R)st->alpha_im;
-  const GenGreen<R> green{ar, ai, ai * ai, a.inv_total};
+  const double kt2 = k1 * k1 + k2 * k2;
+  const double ar = st->alpha_re, ai = st->alpha_im, inv_total = 1.0 / (double)a.N;
+  const GenGreen<R> green{ar, ai, ai * ai, inv_total};
   auto component = [&](int& i, int T) {  // i in [0, C T) -> component, i mod T
     int c = 0;
     if constexpr (C == 3) {
@@ -237,12 +271,13 @@ __global__ void __launch_bounds__(256, GenBounds<R>::min_blocks) k_gen_green(con
   if constexpr (C == 3) {
     // the dyadic split g (F - P_L F) + (i alpha_i / alpha) P_L F (solver.py:571-577, backend/__init__.py:606-649), with
     // the reference's DC rule and no longitudinal part along absent axes
-    const cpx<R> h = divc(mkc<R>((R)0, ai), mkc<R>(ar, ai)) * a.inv_total;
+    const double2 hd = divc(make_double2(0.0, ai), make_double2(ar, ai)) * inv_total;
+    const cpx<R> h = mkc<R>((R)hd.x, (R)hd.y);
     for (int j = slot; j < n; j += nslots) {
-      const R k0 = sk0[j];
-      const R kk2 = k0 * k0 + kt2;
+      const double k0 = sk0[j];
+      const double kk2 = k0 * k0 + kt2;
       const cpx<R> gf = green(kk2);
-      const R kv[3] = {k0, k1, k2};
+      const R kv[3] = {(R)k0, (R)k1, (R)k2};
       cpx<R> F[3], PL[3];
 #pragma unroll
       for (int c = 0; c < 3; ++c) F[c] = cur[((size_t)(c * n + j) << lP) + pl];
@@ -254,7 +289,7 @@ __global__ void __launch_bounds__(256, GenBounds<R>::min_blocks) k_gen_green(con
 #pragma unroll
         for (int c = 0; c < 3; ++c)
           if (c < a.ndim) proj += kv[c] * F[c];
-        proj = proj * ((R)1 / kk2);
+        proj = proj * ((R)1 / (R)kk2);
 #pragma unroll
         for (int c = 0; c < 3; ++c) PL[c] = c < a.ndim ? kv[c] * proj : mkc<R>((R)0, (R)0);
       }
@@ -313,10 +348,9 @@ __global__ void __launch_bounds__(256, GenBounds<R>::min_blocks) k_gen_rows(cons
   const int C = KIND == GEN_ROWS ? 1 : (kPro3 || kEpi3) ? 3 : a.C;
   const int rows = C << lP, pitch = gen_pitch<R>(n);
   const int words = rows * pitch;
-  cpx<R>* sm = reinterpret_cast<cpx<R>*>(mmx_smem_raw);
-  cpx<R>* tw = sm + (size_t)words * ((nst > 2 || kPro3 || kEpi3) ? 2 : 1);
-  const cpx<R>* twg = (const cpx<R>*)a.ax.tw;
-  for (int t = threadIdx.x; t < n; t += blockDim.x) tw[t] = twg[t];
+  gtw<R>* tw = reinterpret_cast<gtw<R>*>(mmx_smem_raw);
+  cpx<R>* sm = reinterpret_cast<cpx<R>*>(tw + n);
+  for (int t = threadIdx.x; t < n; t += blockDim.x) tw[t] = GenTw<R>::load(a.ax, t);
   const int b = blockIdx.y;
   const int64_t row0 = (int64_t)blockIdx.x << lP;
   const int left = a.outer - row0 < P ? (int)(a.outer - row0) : P;  // rows of this tile within the field
