@@ -38,6 +38,7 @@ extern "C" {
 #define MMX_STATUS_OK 0
 #define MMX_STATUS_ZERODIV 1 /* update norm 0 after a previous norm of 0: the reference raises ZeroDivisionError */
 #define MMX_STATUS_TIMEOUT 2 /* a bounded wait for an asynchronous shared-memory copy gave up (results kept valid) */
+#define MMX_STATUS_STALLED 4 /* a bounded wait between the CTAs of one launch gave up (the fields are not valid) */
 
 /*
  * Per right-hand-side iteration state, one entry per batch member, in DEVICE memory.  Mirrors the private state of
@@ -191,6 +192,8 @@ int mmx_pointwise_mul(const void* A, int ra, int ca, const void* B, int cb, int 
 #define MMX_VARIANT_PLANE 8u          /* 3D, 128 x 128 planes, isotropic chi: the two inner axes in one pass */
 #define MMX_VARIANT_FUSED_EPILOGUE 16u /* epilogue fused with the next prologue (speculative); isotropic chi, and a 3x3 chi on 192-sample rows */
 #define MMX_VARIANT_TMA 32u            /* strided 128-sample passes staged by bulk tensor (TMA) copies */
+#define MMX_VARIANT_PASSES 128u        /* one launch per pass also on grids small enough for chunks in one launch */
+#define MMX_VARIANT_LOOP 256u          /* chunks in one launch on any grid that they take */
 #define MMX_VARIANT_RUNTIME_RADIX 64u  /* the runtime-radix passes for lengths without a specialised kernel */
 
 /* Select the kernel variant of a plan (rebuilds its pass list, drops its captured graphs).  No reference

@@ -29,6 +29,7 @@ MMX_ERR_UNSUPPORTED = -3
 MMX_STATUS_OK = 0
 MMX_STATUS_ZERODIV = 1
 MMX_STATUS_TIMEOUT = 2
+MMX_STATUS_STALLED = 4
 MMX_VARIANT_GENERIC = 1
 MMX_VARIANT_SHARED_STAGED = 2
 MMX_VARIANT_PERSISTENT = 4
@@ -36,6 +37,8 @@ MMX_VARIANT_PLANE = 8
 MMX_VARIANT_FUSED_EPILOGUE = 16
 MMX_VARIANT_TMA = 32
 MMX_VARIANT_RUNTIME_RADIX = 64
+MMX_VARIANT_PASSES = 128
+MMX_VARIANT_LOOP = 256
 
 # numpy mirror of struct mmx_rhs_state (include/macromax_b200.h)
 STATE_DTYPE = np.dtype([
@@ -134,6 +137,13 @@ def check(rc: int):
     if rc != MMX_OK:
         msg = _lib.mmx_last_error().decode(errors='replace') if _lib is not None else 'unknown'
         raise NativeError(f'macromax_b200 native call failed ({rc}): {msg}')
+
+
+def check_stalled(states):
+    """Raise when a launch whose blocks wait for one another gave up (MMX_STATUS_STALLED): its fields are not valid."""
+    if np.any(np.asarray(states['status']) & MMX_STATUS_STALLED):
+        raise NativeError('the blocks of an iteration launch did not run together; set another variant '
+                          '(MMX_VARIANT_PASSES) for this plan')
 
 
 def call(name: str, *args):

@@ -112,6 +112,7 @@ class BatchSolution:
         st = self.engine.run(float(rtol), float(maxiter))
         if np.any(st['status'] == nat.MMX_STATUS_ZERODIV):
             raise ZeroDivisionError('float division by zero (update norm after a zero update norm)')
+        nat.check_stalled(st)
         self._state = st
         return self
 

@@ -24,7 +24,7 @@ STAMP = LIB_PATH + '.srchash'
 
 OBJ_DIR = os.path.join(PKG, '_build')
 # compiled side by side and linked into one library; a translation unit whose sources did not change keeps its object
-SOURCES = ['mmx_capi.cu', 'mmx_gen.cu', 'mmx_gen_f64.cu']
+SOURCES = ['mmx_capi.cu', 'mmx_loop.cu', 'mmx_loop_f64.cu', 'mmx_gen.cu', 'mmx_gen_f64.cu']
 NVCC_FLAGS = ['-gencode', 'arch=compute_100a,code=sm_100a', '-lineinfo', '-O3', '-std=c++17',
               '-Xcompiler', '-fPIC', '-Xcompiler', '-O2']
 

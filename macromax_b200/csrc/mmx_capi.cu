@@ -13,6 +13,7 @@
 
 #include "mmx_fast.cuh"
 #include "mmx_gen.h"
+#include "mmx_loop.h"
 #include "mmx_reg.cuh"
 #include "mmx_plane.cuh"
 #include "mmx_epro.cuh"
@@ -140,6 +141,11 @@ struct mmx_plan {
   double* partials = nullptr;
   int64_t partials_len = 0;
   unsigned int* done = nullptr;  // per-RHS tile counters of the epilogue pass (zero between iterations)
+  unsigned int* loop_counter = nullptr;  // the grid barrier of k_loop (two words, zero between launches)
+  LoopCfg loop[3];             // chunks in one launch, per kind of chi (MMX_CHI_SCALAR, MMX_CHI_MAT3, MMX_CHI_SYM6)
+  bool loop_known[3] = {false, false, false};
+  bool passes_only = false;    // MMX_VARIANT_PASSES: no chunks in one launch
+  bool force_loop = false;     // MMX_VARIANT_LOOP: chunks in one launch at any size that they take
   std::vector<PassCfg> iter_passes;
   std::vector<PassCfg> defect_passes;
   bool force_generic = false;  // MMX_FORCE_GENERIC=1: use only the runtime-length kernels (tests)
@@ -153,6 +159,7 @@ struct mmx_plan {
   bool epro = false;           // fuse each epilogue with the next iteration's prologue
   bool tma = false;            // strided 128-sample passes staged by bulk tensor copies (k_tma_pass)
   bool runtime_radix = false;  // k_iter_pass instead of the any-length passes (MMX_VARIANT_RUNTIME_RADIX)
+  bool compare_green = false;  // MMX_WIDE_GREEN set, to 0 or 1: the axis-0 pass's tiles are compared, so it has to run
   bool wide_green = false;     // MMX_WIDE_GREEN=1: 16-pencil tiles for the vector axis-0 pass (tests)
   std::vector<PassCfg> epro_passes;   // [middle passes..., EPI+PRO, repair]; the first PRO runs once per call
   // The last iteration call on this plan whose fused epilogue left the next iteration's first pass (the prologue
@@ -949,6 +956,7 @@ template <class R> IterArgs<R> base_args(mmx_plan* p) {
   a.done = p->done;
   a.l2_window = p->l2_persist ? p->l2_window : 0;
   a.inv_total = (R)(1.0 / (double)p->N);
+  a.inv_total_d = 1.0 / (double)p->N;
   a.poll_limit = p->poll_limit;
   return a;
 }
@@ -958,6 +966,47 @@ bool epro_runs(const mmx_plan* p, int chi_kind) {
   if (p->prec != MMX_C64) return false;
   const bool plane = p->plane && chi_kind == MMX_CHI_SCALAR && !p->plane_passes.empty();
   return !plane && p->epro && epro_serves(p, chi_kind);
+}
+
+// The configuration under which a chunk of iterations runs in one launch, or null.  It does in the default variant where
+// the CTAs can keep the rows of the grid in shared memory (loop_config; up to about 900 000 scalar complex64 samples),
+// except on complex64 grids whose passes are all specialised for their length: those keep the rounding that their other
+// variants and their branch of an uneven batch have, and gain least.  us per iteration, one launch against passes: complex64 300 x 420 15.8 / 30.0, 8 sources
+// on 200 x 180 20.2 / 29.6, 48 x 42 x 44 17.7 / 30.6 (vector: 25.6 / 33.5); specialised: 64^2 8.6 / 13.1, 256^2 12.7 / 18.0,
+// 512^2 22.4 / 24.0, 64^3 20.0 / 18.8; complex128 64^2 8.5 / 20.8, 256^2 11.2 / 32.9, 512^2 23.1 / 29.6, 64^3 27.0 / 34.8;
+// 1000 samples in 1D 7.9 / 20.0 (complex128 8.0 / 24.2).
+const LoopCfg* loop_runs(mmx_plan* p, int chi_kind) {
+  if (p->force_generic || p->no_reg || p->pipe || p->plane || p->epro || p->tma || p->runtime_radix || p->passes_only ||
+      p->compare_green || p->l2_persist)
+    return nullptr;
+  if (p->ncomp == 1 && chi_kind != MMX_CHI_SCALAR) return nullptr;
+  if (p->ndim > 1 && !p->force_loop) {
+    bool special = true;
+    for (const PassCfg& pc : p->iter_passes) special &= pc.fast != 0;
+    if (special) return nullptr;
+  }
+  const int k = chi_kind == MMX_CHI_SCALAR ? 0 : chi_kind == MMX_CHI_MAT3 ? 1 : 2;
+  if (!p->loop_known[k]) {
+    p->loop[k] = p->prec == MMX_C128 ? loop_config<double>(p->ndim, p->shape, p->ncomp, chi_kind, p->batch, sm_count())
+                                     : loop_config<float>(p->ndim, p->shape, p->ncomp, chi_kind, p->batch, sm_count());
+    // the contiguous-axis tiles' partial sums
+    if ((int64_t)p->batch * p->loop[k].tiles[2] * 2 > p->partials_len) p->loop[k].ok = false;
+    p->loop_known[k] = true;
+  }
+  return p->loop[k].ok ? &p->loop[k] : nullptr;
+}
+
+template <class R>
+int run_loop(mmx_plan* p, const LoopCfg& cfg, void* E0, void* E1, const void* chi, int chi_kind, const void* src,
+             mmx_rhs_state* st, int niter, cudaStream_t s) {
+  IterArgs<R> a = base_args<R>(p);
+  a.E0 = (cpx<R>*)E0;
+  a.E1 = (cpx<R>*)E1;
+  a.chi = (const cpx<R>*)chi;
+  a.src = (const cpx<R>*)src;
+  a.st = st;
+  MMX_CUDA(loop_launch<R>(cfg, a, p->ax, p->ncomp, chi_kind, p->batch, niter, p->loop_counter, s));
+  return MMX_OK;
 }
 
 // record the buffers of an iteration call just launched on the stream (the record is cleared unless the call ran
@@ -1234,6 +1283,7 @@ int mmx_plan_create(int ndim, const int64_t* shape, int ncomp, int batch, int pr
     p->pipe = pp && pp[0] == '1';
     const char* wg = getenv("MMX_WIDE_GREEN");
     p->wide_green = wg && wg[0] == '1';
+    p->compare_green = wg && wg[0];
     const char* pl = getenv("MMX_PIPE_POLL_LIMIT");
     if (pl && pl[0]) p->poll_limit = std::max(0, std::min(1 << 20, atoi(pl)));
     const char* lp = getenv("MMX_L2_PERSIST");
@@ -1261,8 +1311,9 @@ int mmx_plan_create(int ndim, const int64_t* shape, int ncomp, int batch, int pr
   for (int i = 0; i < ndim; ++i) maxt = std::max<int64_t>(maxt, p->N / shape[i]);
   p->partials_len = (int64_t)batch * maxt * 2;
   e = cudaMalloc(&p->partials, sizeof(double) * p->partials_len);
-  if (e == cudaSuccess) e = cudaMalloc(&p->done, sizeof(unsigned int) * batch);
-  if (e == cudaSuccess) e = cudaMemset(p->done, 0, sizeof(unsigned int) * batch);
+  if (e == cudaSuccess) e = cudaMalloc(&p->done, sizeof(unsigned int) * (batch + 2));
+  if (e == cudaSuccess) e = cudaMemset(p->done, 0, sizeof(unsigned int) * (batch + 2));
+  p->loop_counter = p->done + batch;
   if (e != cudaSuccess) {
     mmx_plan_destroy(p);
     return cuda_fail(e, "cudaMalloc(partials)");
@@ -1345,6 +1396,11 @@ int mmx_iterate(mmx_plan* p, void* E0, void* E1, const void* chi, int chi_kind, 
   if (niter < 0) return fail(MMX_ERR_ARG, "negative iteration count");
   cudaStream_t s = (cudaStream_t)stream;
   p->cont_valid = false;
+  if (niter > 0) {
+    if (const LoopCfg* loop = loop_runs(p, chi_kind))
+      return p->prec == MMX_C128 ? run_loop<double>(p, *loop, E0, E1, chi, chi_kind, src, state, niter, s)
+                                 : run_loop<float>(p, *loop, E0, E1, chi, chi_kind, src, state, niter, s);
+  }
   const int rc = p->prec == MMX_C128 ? run_iterations<double>(p, E0, E1, chi, chi_kind, src, state, niter, s)
                                      : run_iterations<float>(p, E0, E1, chi, chi_kind, src, state, niter, s);
   if (rc == MMX_OK && niter > 0) note_iteration_call(p, E0, E1, chi, chi_kind, src, state);
@@ -1490,6 +1546,45 @@ int iterate_multi(int n, mmx_plan* const* plans, void* const* E0, void* const* E
     key.ptrs.insert(key.ptrs.end(), {(const void*)p, E0[i], E1[i], chi[i], src[i], (const void*)state[i]});
     key.ints.push_back(chi_kind[i]);
   }
+  // Chunks in one launch need no graph; their CTAs wait for one another, so they run one after another on the stream and
+  // not as branches.  Up to kLoopsInTurn members do so (the fields of a member are those of its own solve); with more, the
+  // branches of passes that run side by side are sooner done.
+  constexpr int kLoopsInTurn = 4;
+  std::vector<int> loops, rest;
+  for (int i = 0; i < n; ++i) (loop_runs(plans[i], chi_kind[i]) ? loops : rest).push_back(i);
+  if (!loops.empty() && (int)loops.size() <= kLoopsInTurn) {
+    if (!rest.empty()) {
+      std::vector<mmx_plan*> rp;
+      std::vector<void*> r0, r1;
+      std::vector<const void*> rc, rs;
+      std::vector<int> rk;
+      std::vector<mmx_rhs_state*> rst;
+      for (int i : rest) {
+        rp.push_back(plans[i]);
+        r0.push_back(E0[i]);
+        r1.push_back(E1[i]);
+        rc.push_back(chi[i]);
+        rk.push_back(chi_kind[i]);
+        rs.push_back(src[i]);
+        rst.push_back(state[i]);
+      }
+      const int code = iterate_multi((int)rest.size(), rp.data(), r0.data(), r1.data(), rc.data(), rk.data(), rs.data(),
+                                     rst.data(), niter, stream, launch, cont);
+      if (code != MMX_OK) return code;
+    }
+    if (!launch) return MMX_OK;
+    for (int i : loops) {
+      mmx_plan* p = plans[i];
+      const LoopCfg& loop = *loop_runs(p, chi_kind[i]);
+      p->cont_valid = false;
+      const cudaStream_t s = (cudaStream_t)stream;
+      const int code = p->prec == MMX_C128
+                           ? run_loop<double>(p, loop, E0[i], E1[i], chi[i], chi_kind[i], src[i], state[i], niter, s)
+                           : run_loop<float>(p, loop, E0[i], E1[i], chi[i], chi_kind[i], src[i], state[i], niter, s);
+      if (code != MMX_OK) return code;
+    }
+    return MMX_OK;
+  }
   key.ints.push_back(niter);
   const bool skip = cont && n == 1 && can_continue(plans[0], E0[0], E1[0], chi[0], chi_kind[0], src[0], state[0]);
   // a prepared continuation also captures the self-contained graph; a launch takes the one that applies
@@ -1548,7 +1643,7 @@ extern "C" int mmx_iterate_graph_continue(mmx_plan* p, void* E0, void* E1, const
 
 extern "C" int mmx_plan_set_variant(mmx_plan* p, unsigned flags) {
   if (!p) return fail(MMX_ERR_ARG, "NULL plan");
-  if (flags & ~127u) return fail(MMX_ERR_ARG, "unknown variant flags");
+  if (flags & ~511u) return fail(MMX_ERR_ARG, "unknown variant flags");
   drop_graphs_of(p);  // captured graphs hold the previous kernels
   p->cont_valid = false;
   p->force_generic = (flags & MMX_VARIANT_GENERIC) != 0;
@@ -1558,6 +1653,8 @@ extern "C" int mmx_plan_set_variant(mmx_plan* p, unsigned flags) {
   p->epro = (flags & MMX_VARIANT_FUSED_EPILOGUE) != 0;
   p->tma = (flags & MMX_VARIANT_TMA) != 0;
   p->runtime_radix = (flags & MMX_VARIANT_RUNTIME_RADIX) != 0;
+  p->passes_only = (flags & MMX_VARIANT_PASSES) != 0;
+  p->force_loop = (flags & MMX_VARIANT_LOOP) != 0;
   p->iter_passes = build_passes(p, false);
   p->defect_passes = build_passes(p, true);
   p->plane_passes = build_plane_passes(p);
@@ -1573,7 +1670,8 @@ extern "C" unsigned mmx_plan_get_variant(const mmx_plan* p) {
   return (p->force_generic ? MMX_VARIANT_GENERIC : 0u) | (p->no_reg ? MMX_VARIANT_SHARED_STAGED : 0u) |
          (p->pipe ? MMX_VARIANT_PERSISTENT : 0u) | (p->plane ? MMX_VARIANT_PLANE : 0u) |
          (p->epro ? MMX_VARIANT_FUSED_EPILOGUE : 0u) | (p->tma ? MMX_VARIANT_TMA : 0u) |
-         (p->runtime_radix ? MMX_VARIANT_RUNTIME_RADIX : 0u);
+         (p->runtime_radix ? MMX_VARIANT_RUNTIME_RADIX : 0u) |
+         (p->passes_only ? MMX_VARIANT_PASSES : 0u) | (p->force_loop ? MMX_VARIANT_LOOP : 0u);
 }
 
 extern "C" int mmx_mat3_extremes(mmx_plan* p, const void* M, int64_t nvox, int mode, double ab, double* out_dev,

@@ -33,6 +33,7 @@ template <class R> struct IterArgs {
   double* partials;      // [B][gridDim.x][2]
   unsigned int* done;    // [B] tiles of the epilogue pass finished (reset by the last one)
   R inv_total;           // 1 / N
+  double inv_total_d;    // the same in FP64
   float2* aux;           // defect output [B][C][N] complex64
   size_t l2_window;      // bytes of T kept L2-resident (0: off); host-side launch attribute only
   int nrhs;              // number of right-hand sides (persistent passes)
@@ -190,6 +191,32 @@ __device__ __forceinline__ void apply_chi2(const float2* __restrict__ chi, int64
   }
 }
 
+// The decision itself, from |d|^2 and |E + d|^2, by one thread.
+static __device__ __forceinline__ void apply_decision(mmx_rhs_state* S, double dd2, double en2) {
+  const double nu = sqrt(dd2);
+  S->iteration += 1;
+  S->last_norm = nu;
+  const double prev = S->prev_norm;
+  if (prev == 0.0) {  // Python float division by zero in solver.py:1079
+    S->status = MMX_STATUS_ZERODIV;
+    S->active = 0;
+    return;
+  }
+  const double rel = nu / prev;
+  if (rel < 1.0) {
+    S->cur ^= 1;
+    S->prev_norm = nu;
+    S->field_norm = sqrt(en2);
+    S->accepted = 1;
+  } else {
+    S->alpha_im = 1.5 * S->alpha_im;  // solver.py:1092
+    S->rejections += 1;
+    S->accepted = 0;
+  }
+  S->residue = S->prev_norm > 0.0 ? S->prev_norm / S->field_norm : 0.0;
+  S->active = ((double)S->iteration < S->maxiter) && (S->residue > S->rtol);
+}
+
 // Accept / reject of Solution.__iter__ (solver.py:1077-1096) and the stop rule of solve (solver.py:81-83,
 // 1112-1121) for one right-hand side, from the epilogue pass partials (deterministic fixed-order reduction).
 // Executed by one whole block.
@@ -227,30 +254,7 @@ static __device__ void decide_rhs(mmx_rhs_state* S, const double* __restrict__ p
   }
   double out2[2];
   block_reduce_2<double>(dd2, en2, out2);
-  if (threadIdx.x == 0) {
-    const double nu = sqrt(out2[0]);
-    S->iteration += 1;
-    S->last_norm = nu;
-    const double prev = S->prev_norm;
-    if (prev == 0.0) {  // Python float division by zero in solver.py:1079
-      S->status = MMX_STATUS_ZERODIV;
-      S->active = 0;
-      return;
-    }
-    const double rel = nu / prev;
-    if (rel < 1.0) {
-      S->cur ^= 1;
-      S->prev_norm = nu;
-      S->field_norm = sqrt(out2[1]);
-      S->accepted = 1;
-    } else {
-      S->alpha_im = 1.5 * S->alpha_im;  // solver.py:1092
-      S->rejections += 1;
-      S->accepted = 0;
-    }
-    S->residue = S->prev_norm > 0.0 ? S->prev_norm / S->field_norm : 0.0;
-    S->active = ((double)S->iteration < S->maxiter) && (S->residue > S->rtol);
-  }
+  if (threadIdx.x == 0) apply_decision(S, out2[0], out2[1]);
 }
 
 // End of the epilogue pass for one tile: publish the tile's partial norms; the last tile of the RHS to finish

@@ -36,26 +36,32 @@ bool best_radices(int n, int stages, int top, int* r, int* sum) {
   return found;
 }
 
-// largest_first: the radices in descending order, else ascending
-bool plan_axis(int n, bool largest_first, GenAxis* ax) {
-  int r[MMX_GEN_STAGES], sum = 0;
-  ax->n = n;
-  ax->nst = 0;
-  for (int stages = 2; stages <= MMX_GEN_STAGES && !ax->nst; ++stages)
-    if (best_radices(n, stages, 16, r, &sum)) ax->nst = stages;
-  if (!ax->nst) return false;
-  if (!largest_first) std::reverse(r, r + ax->nst);
+void fill_axis(int n, int nst, const int* r, GenAxis* ax) {
   auto reciprocal = [](int d) { return d > 1 ? (unsigned)((1ull << 32) / d + 1) : 0u; };
+  *ax = GenAxis();
+  ax->n = n;
+  ax->nst = nst;
   int L = 1;
-  for (int s = 0; s < ax->nst; ++s) {
+  for (int s = 0; s < nst; ++s) {
     ax->r[s] = r[s];
     ax->T[s] = n / r[s];
     ax->L[s] = L;
+    ax->ts[s] = n / r[s] / L;
     ax->mT[s] = reciprocal(ax->T[s]);
     ax->mL[s] = reciprocal(L);
     L *= r[s];
   }
   ax->mn = reciprocal(n);
+}
+
+// largest_first: the radices in descending order, else ascending
+bool plan_axis(int n, bool largest_first, GenAxis* ax) {
+  int r[MMX_GEN_STAGES], sum = 0, nst = 0;
+  for (int stages = 2; stages <= 4 && !nst; ++stages)
+    if (best_radices(n, stages, 16, r, &sum)) nst = stages;
+  if (!nst) return false;
+  if (!largest_first) std::reverse(r, r + nst);
+  fill_axis(n, nst, r, ax);
   return true;
 }
 
@@ -73,6 +79,20 @@ size_t tile_bytes(GenKind kind, const GenAxis& ax, int C, int P, bool dbl) {
 }
 
 }  // namespace
+
+bool gen_small_plan(int n, GenAxis* ax) {
+  int r[MMX_GEN_STAGES], nst = 0, m = n;
+  for (int f : {13, 11, 7, 5, 4, 3, 2})
+    while (m % f == 0 && m > 1) {
+      if (nst == MMX_GEN_STAGES) return false;
+      r[nst++] = f;
+      m /= f;
+    }
+  if (n == 4) nst = 2, r[0] = r[1] = 2;
+  if (m != 1 || nst < 2) return false;
+  fill_axis(n, nst, r, ax);
+  return true;
+}
 
 GenTile gen_tile(GenKind kind, int n, int C, bool dbl, int64_t outer, int64_t inner, int64_t copies, int sms) {
   GenTile t;

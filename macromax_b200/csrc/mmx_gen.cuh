@@ -59,51 +59,71 @@ template <class R> using gtw = typename GenTw<R>::type;
 
 __device__ __forceinline__ unsigned gen_div(unsigned x, unsigned m) { return __umulhi(x, m); }
 
-template <class F> __device__ __forceinline__ void radix_switch(int r, F&& f) {
-  switch (r) {
-    case 2: f(std::integral_constant<int, 2>{}); break;
-    case 3: f(std::integral_constant<int, 3>{}); break;
-    case 4: f(std::integral_constant<int, 4>{}); break;
-    case 5: f(std::integral_constant<int, 5>{}); break;
-    case 6: f(std::integral_constant<int, 6>{}); break;
-    case 7: f(std::integral_constant<int, 7>{}); break;
-    case 8: f(std::integral_constant<int, 8>{}); break;
-    case 9: f(std::integral_constant<int, 9>{}); break;
-    case 10: f(std::integral_constant<int, 10>{}); break;
-    case 11: f(std::integral_constant<int, 11>{}); break;
-    case 12: f(std::integral_constant<int, 12>{}); break;
-    case 13: f(std::integral_constant<int, 13>{}); break;
-    case 14: f(std::integral_constant<int, 14>{}); break;
-    case 15: f(std::integral_constant<int, 15>{}); break;
-    default: f(std::integral_constant<int, 16>{}); break;
+// Radix policies: f(integral_constant<radix>) for the stage's radix.
+struct WideRadices {  // 2 .. 16: few stages, for passes that are bound by traffic
+  template <class F> static __device__ __forceinline__ void run(int r, F&& f) {
+    switch (r) {
+      case 2: f(std::integral_constant<int, 2>{}); break;
+      case 3: f(std::integral_constant<int, 3>{}); break;
+      case 4: f(std::integral_constant<int, 4>{}); break;
+      case 5: f(std::integral_constant<int, 5>{}); break;
+      case 6: f(std::integral_constant<int, 6>{}); break;
+      case 7: f(std::integral_constant<int, 7>{}); break;
+      case 8: f(std::integral_constant<int, 8>{}); break;
+      case 9: f(std::integral_constant<int, 9>{}); break;
+      case 10: f(std::integral_constant<int, 10>{}); break;
+      case 11: f(std::integral_constant<int, 11>{}); break;
+      case 12: f(std::integral_constant<int, 12>{}); break;
+      case 13: f(std::integral_constant<int, 13>{}); break;
+      case 14: f(std::integral_constant<int, 14>{}); break;
+      case 15: f(std::integral_constant<int, 15>{}); break;
+      default: f(std::integral_constant<int, 16>{}); break;
+    }
   }
-}
+};
+struct SmallRadices {  // 4, 5, 3, 2 and the other primes: short butterflies on many threads, for launches bound by latency
+  template <class F> static __device__ __forceinline__ void run(int r, F&& f) {
+    switch (r) {
+      case 2: f(std::integral_constant<int, 2>{}); break;
+      case 3: f(std::integral_constant<int, 3>{}); break;
+      case 4: f(std::integral_constant<int, 4>{}); break;
+      case 5: f(std::integral_constant<int, 5>{}); break;
+      case 7: f(std::integral_constant<int, 7>{}); break;
+      case 11: f(std::integral_constant<int, 11>{}); break;
+      default: f(std::integral_constant<int, 13>{}); break;
+    }
+  }
+};
 
-// Inputs ld(i + q T) of butterfly i, twiddled, and its DFT in u; returns the index of its first output (the others follow
-// at the span L).  FIRST: span 1, no twiddles.
+// Butterfly i of a stage: its inputs ld(q), the samples i + q T, twiddled, and their DFT in u.  Returns the first of its
+// outputs d0 = (i - k) RAD + k, k = i mod L; the others follow at the span L.  FIRST: span 1, no twiddles; ts = T / L.
 template <class R, int RAD, int DIR, bool FIRST, class Ld>
-__device__ __forceinline__ int gen_dft(int i, int T, int L, unsigned mL, const gtw<R>* tw, cpx<R>* u, Ld&& ld) {
+__device__ __forceinline__ int gen_dft(int i, int L, unsigned mL, int ts, const gtw<R>* tw, cpx<R>* u, Ld&& ld) {
 #pragma unroll
-  for (int q = 0; q < RAD; ++q) u[q] = ld(i + q * T);
+  for (int q = 0; q < RAD; ++q) u[q] = ld(q);
   int k = 0;
   if constexpr (!FIRST) {
     if (L > 1) {
       k = i - (int)gen_div((unsigned)i, mL) * L;
-      const int step = k * (int)gen_div((unsigned)T, mL);  // k n / (L RAD)
+      const gtw<R>* w = tw;
+      const int step = k * ts;  // k n / (L RAD)
 #pragma unroll
-      for (int q = 1; q < RAD; ++q) u[q] = GenTw<R>::template mul<DIR>(u[q], tw[q * step]);
+      for (int q = 1; q < RAD; ++q) {
+        w += step;
+        u[q] = GenTw<R>::template mul<DIR>(u[q], *w);
+      }
     }
   }
   gdft<R, RAD, DIR>(u);
   return (i - k) * RAD + k;
 }
+// ... and st(d0, q, value) for the outputs d0 + q L
 template <class R, int RAD, int DIR, bool FIRST, class Ld, class St>
-__device__ __forceinline__ void gen_butterfly(int i, int T, int L, unsigned mL, const gtw<R>* tw, Ld&& ld, St&& st) {
+__device__ __forceinline__ void gen_butterfly(int i, const GenAxis& g, int s, const gtw<R>* tw, Ld&& ld, St&& st) {
   cpx<R> u[RAD];
-  const int d0 = gen_dft<R, RAD, DIR, FIRST>(i, T, L, mL, tw, u, ld);
-  const int Ls = FIRST ? 1 : L;
+  const int d0 = gen_dft<R, RAD, DIR, FIRST>(i, g.L[s], g.mL[s], g.ts[s], tw, u, ld);
 #pragma unroll
-  for (int q = 0; q < RAD; ++q) st(d0 + q * Ls, u[q]);
+  for (int q = 0; q < RAD; ++q) st(d0, q, u[q]);
 }
 
 // -i alpha_i / (|k|^2 - alpha) / N (solver.py:566-568, with the 1/N of the inverse transform), in FP64 and rounded once
@@ -126,102 +146,126 @@ template <class R> struct GenGreen {
   }
 };
 
+// k along the other axes of pencil p of axis 0 (0 beyond the field)
+template <class R>
+__device__ __forceinline__ void gen_pencil_k(const IterArgs<R>& a, unsigned p, double* k1, double* k2) {
+  *k1 = *k2 = 0.0;
+  if (p >= (unsigned)(a.N / a.dims[0])) return;
+  if (a.ndim == 3) {
+    const unsigned i1 = p / (unsigned)a.dims[2];
+    *k1 = a.kvd[1][i1];
+    *k2 = a.kvd[2][p - i1 * (unsigned)a.dims[2]];
+  } else if (a.ndim == 2) {
+    *k1 = a.kvd[1][p];
+  }
+}
+
 // registers: 85 (complex64) and 128 (complex128) per thread at 256 threads
 template <class R> struct GenBounds { static constexpr int min_blocks = sizeof(R) == 4 ? 3 : 2; };
 
+// i alpha_i / (alpha N) (solver.py:575)
+template <class R> __device__ __forceinline__ cpx<R> gen_longitudinal(double ar, double ai, double inv_total) {
+  const double s = ai * inv_total / (ar * ar + ai * ai);
+  return mkc<R>((R)(ai * s), (R)(ar * s));
+}
+
+// The barrier between the stages of a tile: of the whole block, or of the first `threads` threads of it.
+struct BlockSync {
+  __device__ __forceinline__ void operator()() const { __syncthreads(); }
+};
+struct PartSync {
+  int threads;
+  __device__ __forceinline__ void operator()() const { asm volatile("bar.sync 1, %0;" ::"r"(threads) : "memory"); }
+};
+
 // ---------------------------------------------------------------------------------------------------------------
-// Strided axis, FFT only.  blockIdx.y: component plane (right-hand side * C + component), or transform.
+// Strided axis, FFT only: tile `tile` of the component plane `in`, to `out` (may be `in`).  sm: one buffer of P n words,
+// two with more than two stages.  The first barrier publishes tables that the caller has just written.
 // ---------------------------------------------------------------------------------------------------------------
-template <class R, int DIR>
-__global__ void __launch_bounds__(256, GenBounds<R>::min_blocks) k_gen_strided(const __grid_constant__ GenArgs<R> a) {
-  extern __shared__ __align__(16) unsigned char mmx_smem_raw[];
-  const int n = a.g.n, lP = a.lP, P = 1 << lP, nst = a.g.nst;
-  gtw<R>* tw = reinterpret_cast<gtw<R>*>(mmx_smem_raw);
-  cpx<R>* sm = reinterpret_cast<cpx<R>*>(tw + n);
-  for (int t = threadIdx.x; t < n; t += blockDim.x)
-    tw[t] = GenTw<R>::load(a.ax, t);  // published by the first stage's barrier
-  const int pl = threadIdx.x & (P - 1), slot = threadIdx.x >> lP, nslots = blockDim.x >> lP;
-  const unsigned inner = (unsigned)a.inner;
-  const int64_t p = (int64_t)blockIdx.x * P + pl;
-  const bool valid = p < a.outer * a.inner;
+template <class R, int DIR, class Rad, class Sync>
+__device__ __forceinline__ void strided_tile(const GenAxis& g, int lP, unsigned inner, int64_t pencils, int64_t tile,
+                                             const cpx<R>* in, cpx<R>* out, const gtw<R>* tw, cpx<R>* sm, int threads,
+                                             Sync sync) {
+  const int n = g.n, P = 1 << lP, nst = g.nst;
+  const int pl = threadIdx.x & (P - 1), slot = threadIdx.x >> lP, nslots = threads >> lP;
+  const int64_t p = (tile << lP) + pl;
+  const bool valid = p < pencils;
   const int64_t o = p / inner;
-  const int64_t off = (int64_t)blockIdx.y * a.N + o * n * inner + (p - o * inner);
-  pdl_wait();
-  pdl_trigger();
-  if (a.st && !a.st[blockIdx.y / a.C].active) return;
-  const cpx<R>* gi = a.in + off;
-  cpx<R>* go = a.out + off;
-  radix_switch(a.g.r[0], [&](auto rad) {
+  const int64_t off = o * n * inner + (p - o * inner);
+  const cpx<R>* gi = in + off;
+  cpx<R>* go = out + off;
+  Rad::run(g.r[0], [&](auto rad) {
     constexpr int RAD = decltype(rad)::value;
-    const int T = a.g.T[0];
-    for (int i = slot; i < T; i += nslots)
+    const int T = g.T[0];
+    for (int i = slot; i < T; i += nslots) {
+      const cpx<R>* q0 = gi + (size_t)i * inner;
       gen_butterfly<R, RAD, DIR, true>(
-          i, T, 1, 0u, tw, [&](int j) { return valid ? gi[(unsigned)j * inner] : mkc<R>((R)0, (R)0); },
-          [&](int j, cpx<R> v) { sm[(j << lP) + pl] = v; });
+          i, g, 0, tw, [&](int q) { return valid ? q0[(unsigned)(q * T) * inner] : mkc<R>((R)0, (R)0); },
+          [&](int d, int q, cpx<R> v) { sm[((d + q) << lP) + pl] = v; });
+    }
   });
-  __syncthreads();
+  sync();
   cpx<R>* cur = sm;
   for (int s = 1; s + 1 < nst; ++s) {
     cpx<R>* dst = cur == sm ? sm + ((size_t)n << lP) : sm;
-    radix_switch(a.g.r[s], [&](auto rad) {
+    Rad::run(g.r[s], [&](auto rad) {
       constexpr int RAD = decltype(rad)::value;
-      const int T = a.g.T[s];
-      for (int i = slot; i < T; i += nslots)
+      const int T = g.T[s];
+      const int L = g.L[s];
+      for (int i = slot; i < T; i += nslots) {
+        const cpx<R>* q0 = cur + (i << lP) + pl;
         gen_butterfly<R, RAD, DIR, false>(
-            i, T, a.g.L[s], a.g.mL[s], tw, [&](int j) { return cur[(j << lP) + pl]; },
-            [&](int j, cpx<R> v) { dst[(j << lP) + pl] = v; });
+            i, g, s, tw, [&](int q) { return q0[(q * T) << lP]; },
+            [&](int d, int q, cpx<R> v) { dst[((d + q * L) << lP) + pl] = v; });
+      }
     });
-    __syncthreads();
+    sync();
     cur = dst;
   }
   if (!valid) return;
-  radix_switch(a.g.r[nst - 1], [&](auto rad) {
+  Rad::run(g.r[nst - 1], [&](auto rad) {
     constexpr int RAD = decltype(rad)::value;
-    const int T = a.g.T[nst - 1];
-    for (int i = slot; i < T; i += nslots)
+    const int T = g.T[nst - 1];
+    for (int i = slot; i < T; i += nslots) {
+      const cpx<R>* q0 = cur + (i << lP) + pl;
+      cpx<R>* d0 = go + (size_t)i * inner;  // the last stage's outputs are i + q T
       gen_butterfly<R, RAD, DIR, false>(
-          i, T, T, a.g.mL[nst - 1], tw, [&](int j) { return cur[(j << lP) + pl]; },
-          [&](int j, cpx<R> v) { go[(unsigned)j * inner] = v; });
+          i, g, nst - 1, tw, [&](int q) { return q0[(q * T) << lP]; },
+          [&](int, int q, cpx<R> v) { d0[(unsigned)(q * T) * inner] = v; });
+    }
   });
 }
 
-// ---------------------------------------------------------------------------------------------------------------
-// Axis 0: forward FFT, Green multiply, inverse FFT.  blockIdx.y: right-hand side.
-// ---------------------------------------------------------------------------------------------------------------
-template <class R, int C>
-__global__ void __launch_bounds__(256, GenBounds<R>::min_blocks) k_gen_green(const __grid_constant__ GenArgs<R> a) {
+// blockIdx.y: component plane (right-hand side * C + component), or transform.
+template <class R, int DIR>
+__global__ void __launch_bounds__(256, GenBounds<R>::min_blocks) k_gen_strided(const __grid_constant__ GenArgs<R> a) {
   extern __shared__ __align__(16) unsigned char mmx_smem_raw[];
-  const int n = a.g.n, lP = a.lP, P = 1 << lP, nst = a.g.nst;
-  const size_t words = ((size_t)C * n) << lP;
   gtw<R>* tw = reinterpret_cast<gtw<R>*>(mmx_smem_raw);
-  cpx<R>* sm = reinterpret_cast<cpx<R>*>(tw + n);
-  double* sk0 = reinterpret_cast<double*>(sm + 2 * words);  // k of axis 0
-  for (int t = threadIdx.x; t < n; t += blockDim.x) {
-    tw[t] = GenTw<R>::load(a.ax, t);
-    sk0[t] = a.kvd[0][t];
-  }
-  const int b = blockIdx.y;
-  const mmx_rhs_state* st = a.st + b;
-  const int pl = threadIdx.x & (P - 1), slot = threadIdx.x >> lP, nslots = blockDim.x >> lP;
-  const unsigned inner = (unsigned)a.inner;  // axis 0 has outer == 1: a pencil is its inner index
-  const unsigned p = blockIdx.x * P + pl;
-  const bool valid = p < inner;
-  double k1 = 0.0, k2 = 0.0;
-  if (valid) {
-    if (a.ndim == 3) {
-      const unsigned i1 = p / (unsigned)a.dims[2];
-      k1 = a.kvd[1][i1];
-      k2 = a.kvd[2][p - i1 * (unsigned)a.dims[2]];
-    } else if (a.ndim == 2) {
-      k1 = a.kvd[1][p];
-    }
-  }
+  cpx<R>* sm = reinterpret_cast<cpx<R>*>(tw + a.g.n);
+  for (int t = threadIdx.x; t < a.g.n; t += blockDim.x) tw[t] = GenTw<R>::load(a.ax, t);
   pdl_wait();
   pdl_trigger();
-  if (!st->active) return;
-  cpx<R>* g = a.T + (int64_t)b * C * a.N + p;
+  if (a.st && !a.st[blockIdx.y / a.C].active) return;
+  const int64_t plane = (int64_t)blockIdx.y * a.N;
+  strided_tile<R, DIR, WideRadices>(a.g, a.lP, (unsigned)a.inner, a.outer * a.inner, blockIdx.x, a.in + plane, a.out + plane, tw, sm,
+                       blockDim.x, BlockSync());
+}
+
+// ---------------------------------------------------------------------------------------------------------------
+// Axis 0: forward FFT, Green multiply, inverse FFT, in place, of the tile of pencils from tile << lP of one right-hand
+// side (T0: its first component).  h: i alpha_i / (alpha N), the longitudinal factor; sm: two buffers of C P n words; sk0: k of axis 0; k1, k2: of this thread's pencil.
+// ---------------------------------------------------------------------------------------------------------------
+template <class R, int C, class Rad, class Sync>
+__device__ __forceinline__ void green_tile(const GenAxis& g, int lP, int ndim, unsigned inner, int64_t N, unsigned p,
+                                           cpx<R>* T0, double k1, double k2, double ar, double ai, cpx<R> h, double inv_total,
+                                           const gtw<R>* tw,
+                                           const double* sk0, cpx<R>* sm, int threads, Sync sync) {
+  const int n = g.n, P = 1 << lP, nst = g.nst;
+  const size_t words = ((size_t)C * n) << lP;
+  const int pl = threadIdx.x & (P - 1), slot = threadIdx.x >> lP, nslots = threads >> lP;
+  const bool valid = p < inner;  // axis 0 has outer == 1: a pencil is its inner index
+  cpx<R>* gp = T0 + p;
   const double kt2 = k1 * k1 + k2 * k2;
-  const double ar = st->alpha_re, ai = st->alpha_im, inv_total = 1.0 / (double)a.N;
   const GenGreen<R> green{ar, ai, ai * ai, inv_total};
   auto component = [&](int& i, int T) {  // i in [0, C T) -> component, i mod T
     int c = 0;
@@ -231,39 +275,41 @@ __global__ void __launch_bounds__(256, GenBounds<R>::min_blocks) k_gen_green(con
     }
     return c;
   };
-  radix_switch(a.g.r[0], [&](auto rad) {
+  Rad::run(g.r[0], [&](auto rad) {
     constexpr int RAD = decltype(rad)::value;
-    const int T = a.g.T[0];
+    const int T = g.T[0];
     for (int e = slot; e < C * T; e += nslots) {
       int i = e;
       const int c = component(i, T);
-      const cpx<R>* gi = g + (int64_t)c * a.N;
-      cpx<R>* d = sm + (((size_t)c * n) << lP) + pl;
+      const cpx<R>* q0 = gp + (int64_t)c * N + (size_t)i * inner;
+      cpx<R>* o = sm + ((c * n) << lP) + pl;
       gen_butterfly<R, RAD, -1, true>(
-          i, T, 1, 0u, tw, [&](int j) { return valid ? gi[(unsigned)j * inner] : mkc<R>((R)0, (R)0); },
-          [&](int j, cpx<R> v) { d[j << lP] = v; });
+          i, g, 0, tw, [&](int q) { return valid ? q0[(unsigned)(q * T) * inner] : mkc<R>((R)0, (R)0); },
+          [&](int d, int q, cpx<R> v) { o[(d + q) << lP] = v; });
     }
   });
-  __syncthreads();
+  sync();
   cpx<R>*cur = sm, *oth = sm + words;
   for (int s = 1; s < nst; ++s) {
     const bool with_green = C == 1 && s + 1 == nst;
-    radix_switch(a.g.r[s], [&](auto rad) {
+    Rad::run(g.r[s], [&](auto rad) {
       constexpr int RAD = decltype(rad)::value;
-      const int T = a.g.T[s];
+      const int T = g.T[s];
       for (int e = slot; e < C * T; e += nslots) {
         int i = e;
         const int c = component(i, T);
-        const size_t base = (((size_t)c * n) << lP) + pl;
+        const int base = ((c * n) << lP) + pl, L = g.L[s];
+        const cpx<R>* q0 = cur + base + (i << lP);
         gen_butterfly<R, RAD, -1, false>(
-            i, T, a.g.L[s], a.g.mL[s], tw, [&](int j) { return cur[base + (j << lP)]; },
-            [&](int j, cpx<R> v) {
+            i, g, s, tw, [&](int q) { return q0[(q * T) << lP]; },
+            [&](int d, int q, cpx<R> v) {
+              const int j = d + q * L;
               if (with_green) v = v * green(sk0[j] * sk0[j] + kt2);
               oth[base + (j << lP)] = v;
             });
       }
     });
-    __syncthreads();
+    sync();
     cpx<R>* t = cur;
     cur = oth;
     oth = t;
@@ -271,8 +317,6 @@ __global__ void __launch_bounds__(256, GenBounds<R>::min_blocks) k_gen_green(con
   if constexpr (C == 3) {
     // the dyadic split g (F - P_L F) + (i alpha_i / alpha) P_L F (solver.py:571-577, backend/__init__.py:606-649), with
     // the reference's DC rule and no longitudinal part along absent axes
-    const double2 hd = divc(make_double2(0.0, ai), make_double2(ar, ai)) * inv_total;
-    const cpx<R> h = mkc<R>((R)hd.x, (R)hd.y);
     for (int j = slot; j < n; j += nslots) {
       const double k0 = sk0[j];
       const double kk2 = k0 * k0 + kt2;
@@ -283,53 +327,78 @@ __global__ void __launch_bounds__(256, GenBounds<R>::min_blocks) k_gen_green(con
       for (int c = 0; c < 3; ++c) F[c] = cur[((size_t)(c * n + j) << lP) + pl];
       if (j == 0 && p == 0) {
 #pragma unroll
-        for (int c = 0; c < 3; ++c) PL[c] = c < a.ndim ? F[c] : mkc<R>((R)0, (R)0);
+        for (int c = 0; c < 3; ++c) PL[c] = c < ndim ? F[c] : mkc<R>((R)0, (R)0);
       } else {
         cpx<R> proj = mkc<R>((R)0, (R)0);
 #pragma unroll
         for (int c = 0; c < 3; ++c)
-          if (c < a.ndim) proj += kv[c] * F[c];
+          if (c < ndim) proj += kv[c] * F[c];
         proj = proj * ((R)1 / (R)kk2);
 #pragma unroll
-        for (int c = 0; c < 3; ++c) PL[c] = c < a.ndim ? kv[c] * proj : mkc<R>((R)0, (R)0);
+        for (int c = 0; c < 3; ++c) PL[c] = c < ndim ? kv[c] * proj : mkc<R>((R)0, (R)0);
       }
 #pragma unroll
       for (int c = 0; c < 3; ++c) cur[((size_t)(c * n + j) << lP) + pl] = gf * (F[c] - PL[c]) + h * PL[c];
     }
-    __syncthreads();
+    sync();
   }
   for (int s = 0; s + 1 < nst; ++s) {
-    radix_switch(a.g.r[s], [&](auto rad) {
+    Rad::run(g.r[s], [&](auto rad) {
       constexpr int RAD = decltype(rad)::value;
-      const int T = a.g.T[s];
+      const int T = g.T[s];
       for (int e = slot; e < C * T; e += nslots) {
         int i = e;
         const int c = component(i, T);
-        const size_t base = (((size_t)c * n) << lP) + pl;
+        const int base = ((c * n) << lP) + pl, L = g.L[s];
+        const cpx<R>* q0 = cur + base + (i << lP);
         gen_butterfly<R, RAD, +1, false>(
-            i, T, a.g.L[s], a.g.mL[s], tw, [&](int j) { return cur[base + (j << lP)]; },
-            [&](int j, cpx<R> v) { oth[base + (j << lP)] = v; });
+            i, g, s, tw, [&](int q) { return q0[(q * T) << lP]; },
+            [&](int d, int q, cpx<R> v) { oth[base + ((d + q * L) << lP)] = v; });
       }
     });
-    __syncthreads();
+    sync();
     cpx<R>* t = cur;
     cur = oth;
     oth = t;
   }
   if (!valid) return;
-  radix_switch(a.g.r[nst - 1], [&](auto rad) {
+  Rad::run(g.r[nst - 1], [&](auto rad) {
     constexpr int RAD = decltype(rad)::value;
-    const int T = a.g.T[nst - 1];
+    const int T = g.T[nst - 1];
     for (int e = slot; e < C * T; e += nslots) {
       int i = e;
       const int c = component(i, T);
-      const size_t base = (((size_t)c * n) << lP) + pl;
-      cpx<R>* go = g + (int64_t)c * a.N;
+      const cpx<R>* q0 = cur + ((c * n + i) << lP) + pl;
+      cpx<R>* d0 = gp + (int64_t)c * N + (size_t)i * inner;
       gen_butterfly<R, RAD, +1, false>(
-          i, T, T, a.g.mL[nst - 1], tw, [&](int j) { return cur[base + (j << lP)]; },
-          [&](int j, cpx<R> v) { go[(unsigned)j * inner] = v; });
+          i, g, nst - 1, tw, [&](int q) { return q0[(q * T) << lP]; },
+          [&](int, int q, cpx<R> v) { d0[(unsigned)(q * T) * inner] = v; });
     }
   });
+}
+
+// blockIdx.y: right-hand side
+template <class R, int C>
+__global__ void __launch_bounds__(256, GenBounds<R>::min_blocks) k_gen_green(const __grid_constant__ GenArgs<R> a) {
+  extern __shared__ __align__(16) unsigned char mmx_smem_raw[];
+  const int n = a.g.n, P = 1 << a.lP;
+  gtw<R>* tw = reinterpret_cast<gtw<R>*>(mmx_smem_raw);
+  cpx<R>* sm = reinterpret_cast<cpx<R>*>(tw + n);
+  double* sk0 = reinterpret_cast<double*>(sm + 2 * (((size_t)C * n) << a.lP));
+  for (int t = threadIdx.x; t < n; t += blockDim.x) {
+    tw[t] = GenTw<R>::load(a.ax, t);
+    sk0[t] = a.kvd[0][t];
+  }
+  const unsigned p = (blockIdx.x << a.lP) + (threadIdx.x & (P - 1));
+  double k1, k2;
+  gen_pencil_k(a, p, &k1, &k2);
+  pdl_wait();
+  pdl_trigger();
+  const mmx_rhs_state* st = a.st + blockIdx.y;
+  if (!st->active) return;
+  green_tile<R, C, WideRadices>(a.g, a.lP, a.ndim, (unsigned)a.inner, a.N, p, a.T + (int64_t)blockIdx.y * C * a.N, k1, k2,
+                   st->alpha_re, st->alpha_im, gen_longitudinal<R>(st->alpha_re, st->alpha_im, a.inv_total_d), a.inv_total_d,
+                   tw, sk0, sm, blockDim.x, BlockSync());
 }
 
 // ---------------------------------------------------------------------------------------------------------------
@@ -395,7 +464,7 @@ __global__ void __launch_bounds__(256, GenBounds<R>::min_blocks) k_gen_rows(cons
     }
     __syncthreads();
   } else {
-    radix_switch(a.g.r[0], [&](auto rad) {
+    WideRadices::run(a.g.r[0], [&](auto rad) {
       constexpr int RAD = decltype(rad)::value;
       const int T = a.g.T[0];
       for (int e = threadIdx.x; e < rows * T; e += blockDim.x) {
@@ -407,18 +476,19 @@ __global__ void __launch_bounds__(256, GenBounds<R>::min_blocks) k_gen_rows(cons
           const cpx<R>*eS = Ecur + off, *sS = S + off, *xS = X + (int64_t)(r & (P - 1)) * n;
           const bool with_src = !source_is_zero(st, r >> lP);
           gen_butterfly<R, RAD, DIR, true>(
-              i, T, 1, 0u, tw,
-              [&](int j) {
+              i, a.g, 0, tw,
+              [&](int q) {
+                const int j = i + q * T;
                 cpx<R> v = (cc.a * xS[j] + cc.b) * eS[j];
                 if (with_src) v += cc.s * sS[j];
                 return v;
               },
-              [&](int j, cpx<R> v) { d[gen_at<R>(j)] = v; });
+              [&](int o, int q, cpx<R> v) { d[gen_at<R>(o + q)] = v; });
         } else {
-          const cpx<R>* tS = gi + off;
+          const cpx<R>* tS = gi + off + i;
           gen_butterfly<R, RAD, DIR, true>(
-              i, T, 1, 0u, tw, [&](int j) { return KIND == GEN_ROWS ? tS[j] * a.scale : tS[j]; },
-              [&](int j, cpx<R> v) { d[gen_at<R>(j)] = v; });
+              i, a.g, 0, tw, [&](int q) { return KIND == GEN_ROWS ? tS[q * T] * a.scale : tS[q * T]; },
+              [&](int o, int q, cpx<R> v) { d[gen_at<R>(o + q)] = v; });
         }
       }
     });
@@ -428,16 +498,17 @@ __global__ void __launch_bounds__(256, GenBounds<R>::min_blocks) k_gen_rows(cons
   const int s1 = kEpi3 ? nst : nst - 1;  // the stages between shared-memory buffers
   for (int s = s0; s < s1; ++s) {
     cpx<R>* dst = cur == sm ? sm + words : sm;
-    radix_switch(a.g.r[s], [&](auto rad) {
+    WideRadices::run(a.g.r[s], [&](auto rad) {
       constexpr int RAD = decltype(rad)::value;
       const int T = a.g.T[s];
       for (int e = threadIdx.x; e < rows * T; e += blockDim.x) {
         const int r = (int)gen_div((unsigned)e, a.g.mT[s]), i = e - r * T;
         const cpx<R>* src = cur + r * pitch;
         cpx<R>* d = dst + r * pitch;
+        const int L = a.g.L[s];
         gen_butterfly<R, RAD, DIR, false>(
-            i, T, a.g.L[s], a.g.mL[s], tw, [&](int j) { return src[gen_at<R>(j)]; },
-            [&](int j, cpx<R> v) { d[gen_at<R>(j)] = v; });
+            i, a.g, s, tw, [&](int q) { return src[gen_at<R>(i + q * T)]; },
+            [&](int o, int q, cpx<R> v) { d[gen_at<R>(o + q * L)] = v; });
       }
     });
     __syncthreads();
@@ -479,7 +550,7 @@ __global__ void __launch_bounds__(256, GenBounds<R>::min_blocks) k_gen_rows(cons
       }
     }
   } else {
-    radix_switch(a.g.r[nst - 1], [&](auto rad) {
+    WideRadices::run(a.g.r[nst - 1], [&](auto rad) {
       constexpr int RAD = decltype(rad)::value;
       const int T = a.g.T[nst - 1];
       for (int e = threadIdx.x; e < rows * T; e += blockDim.x) {
@@ -491,7 +562,7 @@ __global__ void __launch_bounds__(256, GenBounds<R>::min_blocks) k_gen_rows(cons
           const cpx<R>*eS = Ecur + off, *xS = X + (int64_t)(r & (P - 1)) * n;
           cpx<R>* eO = Eoth + off;
           cpx<R> u[RAD];
-          gen_dft<R, RAD, DIR, false>(i, T, T, a.g.mL[nst - 1], tw, u, [&](int j) { return src[gen_at<R>(j)]; });
+          gen_dft<R, RAD, DIR, false>(i, T, a.g.mL[nst - 1], 1, tw, u, [&](int q) { return src[gen_at<R>(i + q * T)]; });
           // the outputs at i + q T: E and chi of CH of them are in flight at a time
           constexpr int CH = RAD <= 8 ? RAD : (RAD + 1) / 2;
 #pragma unroll
@@ -514,10 +585,10 @@ __global__ void __launch_bounds__(256, GenBounds<R>::min_blocks) k_gen_rows(cons
               }
           }
         } else {
-          cpx<R>* tO = go + off;
+          cpx<R>* tO = go + off + i;
           gen_butterfly<R, RAD, DIR, false>(
-              i, T, T, a.g.mL[nst - 1], tw, [&](int j) { return src[gen_at<R>(j)]; },
-              [&](int j, cpx<R> v) { tO[j] = v; });
+              i, a.g, nst - 1, tw, [&](int q) { return src[gen_at<R>(i + q * T)]; },
+              [&](int, int q, cpx<R> v) { tO[q * T] = v; });
         }
       }
     });

@@ -5,14 +5,14 @@
 
 #include "mmx_device.cuh"
 
-#define MMX_GEN_STAGES 4
+#define MMX_GEN_STAGES 8
 
 // Radix plan of one axis: stage s has radix r[s], T[s] = n / r[s] butterflies per pencil and span L[s] (the product of
 // the radices before it); m* are the multipliers of the exact division x / d = (x m) >> 32, m = 2^32 / d + 1, valid for
 // x d < 2^32.
 struct GenAxis {
   int n, nst;
-  int r[MMX_GEN_STAGES], T[MMX_GEN_STAGES], L[MMX_GEN_STAGES];
+  int r[MMX_GEN_STAGES], T[MMX_GEN_STAGES], L[MMX_GEN_STAGES], ts[MMX_GEN_STAGES];  // ts = T / L
   unsigned mT[MMX_GEN_STAGES], mL[MMX_GEN_STAGES], mn;
 };
 
@@ -33,6 +33,9 @@ struct GenTile {
   size_t smem = 0;
   int64_t tiles = 0;
 };
+
+// The plan of an axis for launches bound by latency: radices 4, 5, 3, 2, 7, 11, 13.
+bool gen_small_plan(int n, GenAxis* ax);
 
 // Tile of a pass over `outer * inner` pencils of n samples for C components (GEN_STRIDED, GEN_ROWS: C = 1); copies: the
 // number of independent such passes in one launch (right-hand sides, or components of them).

@@ -132,6 +132,7 @@ class MixedSolution:
                  _ptr(eng.state), _ptr(eng.sources), _stream())
         eng.iterate(1)  # first correction step: its update norm is ||d(x)||
         st = eng.read_state()
+        nat.check_stalled(st)
         res = np.full(self.batch, np.inf)
         xn = self._xnorms()
         pos = xn > 0
@@ -153,6 +154,7 @@ class MixedSolution:
         """x += delta for every right-hand side that was still correcting."""
         eng = self.inner.engine
         st = eng.read_state()
+        nat.check_stalled(st)
         self.inner_iterations.append(st['iteration'].copy())
         for b in range(self.batch):  # x += delta from the current buffer of each right-hand side (no gather)
             if not self._done[b]:

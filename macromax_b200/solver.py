@@ -318,6 +318,7 @@ class Solution:
     def _check_status(self, st):
         if int(st['status']) == nat.MMX_STATUS_ZERODIV:
             raise ZeroDivisionError('float division by zero (update norm after a zero update norm)')
+        nat.check_stalled(st)
 
     # -- iteration --------------------------------------------------------------------------------------------------
     def __iter__(self):

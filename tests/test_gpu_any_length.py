@@ -1,7 +1,8 @@
 """
-The passes for axes of any length (complex64 lengths without a specialised kernel, and complex128) against the
-runtime-radix kernels and the numpy oracle: every radix up to 16, two to four stages, ragged last tiles, scalar and
-vector fields, isotropic, symmetric and general 3x3 permittivities, batches; and the transforms against numpy.
+The passes for axes of any length (complex64 lengths without a specialised kernel, and complex128), launched one by one
+and as chunks of iterations in one launch, against the runtime-radix kernels and the numpy oracle: every radix up to 16,
+two to four stages, ragged last tiles, scalar and vector fields, isotropic, symmetric and general 3x3 permittivities,
+batches, rejected updates; and the transforms against numpy.
 """
 import numpy as np
 import pytest
@@ -38,10 +39,13 @@ CASES = [((22, 26), 1, 'scalar'), ((300, 420), 1, 'scalar'), ((9, 1500), 1, 'sca
 
 @pytest.mark.parametrize('shape,components,medium', CASES)
 @pytest.mark.parametrize('dtype', [np.complex64, np.complex128])
-def test_iteration_matches_generic_and_oracle(shape, components, medium, dtype):
+@pytest.mark.parametrize('launches', ['passes', 'loop'])
+def test_iteration_matches_generic_and_oracle(shape, components, medium, dtype, launches):
+    from macromax_b200 import _native as nat, autotune
     from oracle import mmoracle as mo
     wl = _problem(shape, components, medium)
     fast, gen = _solution(wl, dtype), _solution(wl, dtype, generic=True)
+    autotune.set_variant(fast._engine, nat.MMX_VARIANT_PASSES if launches == 'passes' else nat.MMX_VARIANT_LOOP)
     ref = mo.from_workload(wl, np.complex128)
     assert abs(fast.alpha - ref.alpha) <= 1e-9 * abs(ref.alpha)
     for s in (fast, gen):
@@ -53,6 +57,42 @@ def test_iteration_matches_generic_and_oracle(shape, components, medium, dtype):
     assert rel(fast.E, gen.E) < tol
     assert rel(fast.E, ref.E) < max(tol, 1e-9 if medium != 'scalar' else 0)  # a 3x3 alpha: closed-form eigenvalues
     assert fast.residue == pytest.approx(gen.residue, rel=10 * tol)
+
+
+@pytest.mark.parametrize('shape,components', [((1000,), 1), ((77,), 3), ((4,), 1), ((2160,), 1), ((825,), 3)])
+@pytest.mark.parametrize('dtype', [np.complex64, np.complex128])
+def test_line_matches_generic_and_oracle(shape, components, dtype):
+    from oracle import mmoracle as mo
+    wl = _problem(shape, components, 'scalar')
+    wl['bound_thickness'] = 0.0 if shape[0] < 8 else wl['bound_thickness']
+    fast, gen = _solution(wl, dtype), _solution(wl, dtype, generic=True)
+    ref = mo.from_workload(wl, np.complex128)
+    for s in (fast, gen):
+        s.solve(None, rtol=0, maxiter=20)
+    ref.solve(rtol=0, maxiter=20)
+    assert fast.iteration == gen.iteration == 20
+    tol = 1e-5 if dtype == np.complex64 else 1e-12
+    assert rel(fast.E, gen.E) < tol
+    assert rel(fast.E, ref.E) < tol
+
+
+@pytest.mark.parametrize('shape,components', [((300,), 1), ((44, 60), 1), ((18, 20, 22), 1), ((40, 36), 3)])
+@pytest.mark.parametrize('launches', ['passes', 'loop'])
+def test_rejected_updates_match_generic(shape, components, launches):
+    """A medium with gain: the divergence guard rejects updates; alpha, the rejections and the field are the same."""
+    from macromax_b200 import _native as nat, autotune
+    wl = _problem(shape, components, 'scalar')
+    rng = np.random.default_rng(9)
+    wl['epsilon'] = wl['epsilon'] - 0.45j * rng.uniform(size=shape)
+    wl['bound_thickness'] = 0.0
+    fast, gen = _solution(wl, np.complex128), _solution(wl, np.complex128, generic=True)
+    autotune.set_variant(fast._engine, nat.MMX_VARIANT_PASSES if launches == 'passes' else nat.MMX_VARIANT_LOOP)
+    for s in (fast, gen):
+        s.solve(None, rtol=0, maxiter=25)
+    assert gen.rejections > 0
+    assert (fast.rejections, fast.iteration) == (gen.rejections, gen.iteration)
+    assert fast.alpha == pytest.approx(gen.alpha, rel=1e-14)
+    assert rel(fast.E, gen.E) < 1e-9  # updates of a nearly diverging iteration
 
 
 @pytest.mark.parametrize('shape,components,batch', [((60, 77), 1, 5), ((20, 18, 26), 3, 3), ((96, 10), 1, 40)])
