@@ -185,6 +185,10 @@ int mmx_adjoint_grad(const void* E, const void* nu, void* grad, int64_t batch, i
 int mmx_pointwise_mul(const void* A, int ra, int ca, const void* B, int cb, int b_broadcast, void* out,
                       int64_t nvox, int precision, void* stream);
 
+/* 1 when a chunk of iterations of this plan runs in one launch that ends when no right-hand side is active any more, so
+ * that a chunk longer than the solve costs nothing; 0 when every iteration is launched (and may leave at once). */
+int mmx_plan_chunk_ends(mmx_plan* plan, int chi_kind);
+
 /* Kernel variants of a plan (bit flags), chosen by the autotuner (macromax_b200/autotune.py). */
 #define MMX_VARIANT_GENERIC 1u        /* runtime-length shared-memory kernels only */
 #define MMX_VARIANT_SHARED_STAGED 2u  /* compile-time kernels without the register-staged passes */

@@ -1665,6 +1665,11 @@ extern "C" int mmx_plan_set_variant(mmx_plan* p, unsigned flags) {
   return MMX_OK;
 }
 
+extern "C" int mmx_plan_chunk_ends(mmx_plan* p, int chi_kind) {
+  if (!p || (chi_kind != MMX_CHI_SCALAR && chi_kind != MMX_CHI_MAT3 && chi_kind != MMX_CHI_SYM6)) return 0;
+  return loop_runs(p, chi_kind) != nullptr;
+}
+
 extern "C" unsigned mmx_plan_get_variant(const mmx_plan* p) {
   if (!p) return 0u;
   return (p->force_generic ? MMX_VARIANT_GENERIC : 0u) | (p->no_reg ? MMX_VARIANT_SHARED_STAGED : 0u) |

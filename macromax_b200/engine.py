@@ -8,6 +8,7 @@ only edits the small state array between calls (reset of the update norm, stop r
 """
 from __future__ import annotations
 
+import threading
 
 import numpy as np
 import torch
@@ -73,6 +74,9 @@ class IterationEngine:
             self.fields = torch.zeros((2, self.batch, self.ncomp, self.N), dtype=self.torch_dtype, device=self.device)
             self.sources = torch.zeros((self.batch, self.ncomp, self.N), dtype=self.torch_dtype, device=self.device)
             self.state = torch.zeros((self.batch, nat.STATE_DTYPE.itemsize), dtype=torch.uint8, device=self.device)
+        self._state_host = torch.empty(self.state.shape, dtype=torch.uint8, pin_memory=True)
+        self._state_lock = threading.Lock()
+        self._launches = 0  # iteration calls so far: with the state tensor's version, what a copy of the state is of
         self.set_chi(chi0, alpha0)
         st = np.zeros(self.batch, dtype=nat.STATE_DTYPE)
         st['alpha_re'] = st['alpha0_re'] = alpha0.real
@@ -148,12 +152,18 @@ class IterationEngine:
 
     # -- state ------------------------------------------------------------------------------------------------------
     def read_state(self) -> np.ndarray:
-        raw = self.state.cpu().numpy()
-        return raw.view(nat.STATE_DTYPE).reshape(self.batch).copy()
+        with self._state_lock:  # one staging buffer
+            self._state_host.copy_(self.state, non_blocking=True)
+            torch.cuda.current_stream(self.device).synchronize()
+            return self._state_host.numpy().view(nat.STATE_DTYPE).reshape(self.batch).copy()
+
+    def state_key(self):
+        """Changes with every iteration call and with every write to the state tensor."""
+        return self._launches, self.state._version
 
     def write_state(self, st: np.ndarray):
         raw = np.ascontiguousarray(st, dtype=nat.STATE_DTYPE).view(np.uint8).reshape(self.batch, -1)
-        self.state.copy_(torch.from_numpy(raw.copy()).to(self.device))
+        self.state.copy_(torch.from_numpy(raw.copy()))
 
     def reset_alpha(self, index=None):
         """Return alpha to alpha0 (the stored chi and sources), e.g. before solving a new, unrelated problem."""
@@ -193,13 +203,15 @@ class IterationEngine:
     # -- iteration --------------------------------------------------------------------------------------------------
     use_graphs = True  # replay captured CUDA graphs for multi-iteration chunks
 
-    def iterate(self, niter: int, stream=None, cont: bool = False):
+    def iterate(self, niter: int, stream=None, cont: bool = False, graph: bool = True):
         """``niter`` iterations on the stream.  cont: the next chunk of the same solve -- nothing has written the
         fields, chi, sources or states since the previous call -- so the chunk may start from the first pass that
-        the previous chunk's fused epilogue left in the work buffer (mmx_iterate_graph_continue)."""
+        the previous chunk's fused epilogue left in the work buffer (mmx_iterate_graph_continue).  graph: replay a captured
+        graph of ``niter`` iterations (a length that comes again)."""
         if niter <= 0:
             return
-        if self.use_graphs and niter > 1:
+        self._launches += 1
+        if self.use_graphs and niter > 1 and graph:
             fn = 'mmx_iterate_graph_continue' if cont else 'mmx_iterate_graph'
         else:
             fn = 'mmx_iterate'
@@ -211,11 +223,16 @@ class IterationEngine:
         nat.call('mmx_iterate_graph_prepare', self.plan.handle, _ptr(self.fields[0]), _ptr(self.fields[1]),
                  _ptr(self.chi), self.chi_kind, _ptr(self.sources), _ptr(self.state), int(niter))
 
-    def run(self, rtol: float, maxiter: float, chunk: int = 8, max_chunk: int = 64,
+    def run(self, rtol: float, maxiter: float, chunk: int = 16, max_chunk: int = 64,
             reset_iteration: bool = True) -> np.ndarray:
         """Iterate every active RHS until its stop rule (iteration < maxiter and residue > rtol) fails; the iteration
         count starts from 0 (as every Solution.solve, solver.py:1063), or goes on from its current value
-        (reset_iteration=False)."""
+        (reset_iteration=False).
+
+        The device stops by itself; the host looks at the states after ``chunk`` iterations, then after twice as many,
+        and so on up to ``max_chunk``, and asks for no more than ``maxiter`` of them.  Where a launch runs a whole chunk
+        and ends with the solve, a chunk is a long one; elsewhere all chunks replay one graph of ``chunk`` iterations, the
+        only one that a solve of a new problem captures."""
         st = self.read_state()
         if reset_iteration:
             st['iteration'] = 0
@@ -225,13 +242,22 @@ class IterationEngine:
         st['status'] = 0
         self.write_state(st)
         cont = False  # the chunks after the first continue the same solve (the loop only reads the state)
+        whole = bool(nat.load().mmx_plan_chunk_ends(self.plan.handle, self.chi_kind))
+        look = max(512, max_chunk) if whole else chunk
+        if rtol <= 0 and not whole:
+            look = max(chunk, max_chunk)  # nothing to stop for before maxiter
         while True:
-            self.iterate(chunk, cont=cont)
-            cont = True
+            left = maxiter - float(np.min(st['iteration'][st['active'] != 0]))
+            todo = int(min(look, max(left, 1)))
+            while todo > 0:
+                n = todo if whole else min(todo, chunk)
+                self.iterate(n, cont=cont, graph=whole or n == chunk)
+                cont = True
+                todo -= n
             st = self.read_state()
             if not np.any(st['active']):
                 break
-            chunk = min(chunk * 2, max_chunk)
+            look = look if whole else min(look * 2, max_chunk)
         return st
 
     def to_host(self, t: torch.Tensor) -> np.ndarray:

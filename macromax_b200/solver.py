@@ -123,6 +123,7 @@ class Solution:
                 chi_b = np.eye(3).reshape(3, 3, *([1] * self._grid.ndim)) * chi_b
             epsilon = epsilon + chi_b
         self._engine = None
+        self._snapshot = None
         self._device = device
         self._prepare(epsilon, source_distribution, initial_field)
 
@@ -159,6 +160,11 @@ class Solution:
 
     @property
     def _state(self):
+        # between two iterations (a callback's iteration, residue, ...) the state that the last one was checked by serves,
+        # unless the device's has been written since
+        snap = self._snapshot
+        if snap is not None and snap[0] == self._engine.state_key():
+            return snap[1]
         return self._engine.read_state()[0]
 
     # -- properties of the reference API ----------------------------------------------------------------------------
@@ -334,7 +340,9 @@ class Solution:
         self._engine.write_state(st)
         while True:
             self._engine.iterate(1)
-            self._check_status(self._state)
+            st = self._engine.read_state()[0]
+            self._snapshot = (self._engine.state_key(), st)
+            self._check_status(st)
             yield self
 
     def solve(self, callback: Callable[['Solution'], bool] | None = _default_callback, rtol: float = 0,
