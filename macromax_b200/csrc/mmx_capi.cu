@@ -961,11 +961,21 @@ template <class R> IterArgs<R> base_args(mmx_plan* p) {
   return a;
 }
 
+// The fused-epilogue schedule is chosen by its variant flag, and in the default variant for 3-component fields on 3D grids
+// (us per iteration, plain and fused: 64^3 28.7 / 26.5, four sources 66.7 / 63.5; 128^3 119.7 / 109.5, four sources 482 /
+// 462; 192^3 with a 3x3 chi 555 / 490).  On 2D grids and for scalar fields it is not faster (128^3 scalar 47.1 / 50.5, 64
+// sources on 512^2 264 / 297): their passes hold less work per sample to hide its longer dependent chain behind.
+bool epro_chosen(const mmx_plan* p) {
+  if (p->epro) return true;
+  return p->ncomp == 3 && p->ndim == 3 && !p->force_generic && !p->no_reg && !p->pipe && !p->plane &&
+         !p->runtime_radix && !p->passes_only && !p->compare_green && !p->l2_persist;
+}
+
 // whether run_iterations takes the fused-epilogue schedule for this plan and chi
 bool epro_runs(const mmx_plan* p, int chi_kind) {
   if (p->prec != MMX_C64) return false;
   const bool plane = p->plane && chi_kind == MMX_CHI_SCALAR && !p->plane_passes.empty();
-  return !plane && p->epro && epro_serves(p, chi_kind);
+  return !plane && epro_chosen(p) && epro_serves(p, chi_kind);
 }
 
 // The configuration under which a chunk of iterations runs in one launch, or null.  It does in the default variant where
@@ -1042,7 +1052,7 @@ int run_iterations(mmx_plan* p, void* E0, void* E1, const void* chi, int chi_kin
   // the accept/reject decision is taken by the last tile of the epilogue pass (no separate launch)
   const bool plane = std::is_same<R, float>::value && p->plane && chi_kind == MMX_CHI_SCALAR &&
                      !p->plane_passes.empty();
-  const bool epro = std::is_same<R, float>::value && !plane && p->epro && epro_serves(p, chi_kind);
+  const bool epro = std::is_same<R, float>::value && !plane && epro_chosen(p) && epro_serves(p, chi_kind);
   if (epro) {
     // first prologue of the chunk, then per iteration the middle passes, the fused epilogue + next prologue and
     // the repair pass
