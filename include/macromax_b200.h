@@ -224,6 +224,8 @@ int mmx_mat3_extremes(mmx_plan* plan, const void* M, int64_t nvox, int mode, dou
  * composed on the host from mmx_fftn and these kernels.  Fields are [3][N] in the plan's precision; k are the plan's
  * k-vectors (mmx_plan_set_kvectors, k0-scaled grid).
  *   mmx_curl_ft:  out = i k x F for a spectrum F (not in place).            Replaces BackEnd.curl_ft (:483-509).
+ *   mmx_project_ft: the longitudinal part of a spectrum F, or (transversal != 0) F minus it; out may be F.
+ *                 Replaces longitudinal_ / transversal_projection_ft (backend/__init__.py:606-649).
  *   mmx_green_ft: F <- g (F - P_L F) + (i alpha_i / alpha) P_L F in place,   Replaces g_ft_op (solver.py:571-577).
  *                 g = -i alpha_i / (|k|^2 - alpha); no 1/N (the inverse mmx_fftn scales).
  *   mmx_chi_mix:  u = (a chi_EE0 + b I) x + f_HE chi_HE0 d, w = f_EH chi_EH0 x + f_HH chi_HH0 d per voxel, the four
@@ -232,6 +234,7 @@ int mmx_mat3_extremes(mmx_plan* plan, const void* M, int64_t nvox, int mode, dou
  *                 __update_operators (solver.py:514-528).
  *   mmx_axpby:    out = a x + b y (nwords complex words).
  */
+int mmx_project_ft(mmx_plan* plan, const void* F, void* out, int transversal, void* stream);
 int mmx_curl_ft(mmx_plan* plan, const void* F, void* out, void* stream);
 int mmx_green_ft(mmx_plan* plan, void* F, double alpha_re, double alpha_im, void* stream);
 int mmx_chi_mix(const void* x, const void* d, const void* chi_ee, const void* chi_eh, const void* chi_he,

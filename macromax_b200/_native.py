@@ -109,6 +109,7 @@ def load(path: str | None = None):
         'mmx_scalar_sigma': (i32, [vp, vp, i64, dbl, vp, vp]),
         'mmx_chi_from_eps': (i32, [vp, i32, i64, dbl, dbl, dbl, dbl, vp, i32, vp]),
         'mmx_magnetic_iterate': (i32, [vp, ctypes.POINTER(MagneticBuffers), vp, i32, i32, vp]),
+        'mmx_project_ft': (i32, [vp, vp, vp, i32, vp]),
         'mmx_curl_ft': (i32, [vp, vp, vp, vp]),
         'mmx_green_ft': (i32, [vp, vp, dbl, dbl, vp]),
         'mmx_chi_mix': (i32, [vp, vp, vp, vp, vp, vp, ctypes.POINTER(dbl), vp, vp, i64, i32, vp]),

@@ -292,10 +292,26 @@ class BackEndB200:
             self._k2 = sum(k ** 2 for k in self.k)
         return self._k2
 
+    def _project(self, F, transversal: bool):
+        """The projection of a 3-component field of this grid by mmx_project_ft; None for other shapes and for tensors
+        whose derivatives or batching torch tracks."""
+        if tuple(F.shape) != (3, 1, *(int(n) for n in self._grid.shape)) or F.requires_grad or \
+                torch._C._functorch.is_functorch_wrapped_tensor(F) or \
+                torch.autograd.forward_ad.unpack_dual(F).tangent is not None:
+            return None
+        x = F.resolve_conj().resolve_neg().contiguous()
+        out = torch.empty_like(x)
+        nat.call('mmx_project_ft', self._plan.handle, _ptr(x), _ptr(out), int(transversal), _stream())
+        return out
+
     def longitudinal_projection_ft(self, F):
-        """backend/__init__.py:606-649 (DC passed through, components >= ndim zero); a per-op tensor expression (the
-        fused iteration applies the projection inside its axis-0 pass)."""
+        """backend/__init__.py:606-649 (DC passed through, components >= ndim zero); a 3-component field of this grid in
+        one kernel, other shapes as tensor expressions (the fused iteration applies the projection inside its axis-0
+        pass)."""
         F = self.astype(F)
+        out = self._project(F, False)
+        if out is not None:
+            return out
         nd = self._grid.ndim
         proj = F[0, 0] * self.k[0]
         for a in range(1, nd):
@@ -313,7 +329,8 @@ class BackEndB200:
 
     def transversal_projection_ft(self, F):
         F = self.astype(F)
-        return F - self.longitudinal_projection_ft(F)
+        out = self._project(F, True)
+        return out if out is not None else F - self.longitudinal_projection_ft(F)
 
     def curl_ft(self, F):
         """backend/__init__.py:483-509: i k x F.  A 3-component field of this grid goes through mmx_curl_ft."""

@@ -1717,6 +1717,26 @@ template <class R> const R* kv_of(const mmx_plan* p, int axis) {
 }
 }  // namespace
 
+extern "C" int mmx_project_ft(mmx_plan* p, const void* F, void* out, int transversal, void* stream) {
+  if (!p || !F || !out) return fail(MMX_ERR_ARG, "NULL plan or buffer");
+  if (!p->kv_set) return fail(MMX_ERR_ARG, "k-vectors not set (mmx_plan_set_kvectors)");
+  const KGrid g = kgrid_of(p);
+  const int n = (int)p->shape[p->ndim - 1];
+  const dim3 block(n <= 32 ? 32 : n <= 64 ? 64 : 128, n <= 32 ? 8 : n <= 64 ? 4 : 2);
+  const int64_t rows = p->N / n;
+  const unsigned blocks = (unsigned)std::min<int64_t>((rows + block.y - 1) / block.y, (int64_t)sm_count() * 32);
+  const double* k = p->prec == MMX_C128 ? (const double*)p->kv_dev : p->kvd_dev;
+  const double* kv[3] = {k + p->kv_off[0], p->ndim > 1 ? k + p->kv_off[1] : nullptr, p->ndim > 2 ? k + p->kv_off[2] : nullptr};
+  if (p->prec == MMX_C128)
+    k_project_ft<double><<<blocks, block, 0, (cudaStream_t)stream>>>((const double2*)F, (double2*)out, g, kv[0], kv[1],
+                                                                     kv[2], transversal);
+  else
+    k_project_ft<float><<<blocks, block, 0, (cudaStream_t)stream>>>((const float2*)F, (float2*)out, g, kv[0], kv[1], kv[2],
+                                                                    transversal);
+  MMX_CUDA(cudaGetLastError());
+  return MMX_OK;
+}
+
 extern "C" int mmx_curl_ft(mmx_plan* p, const void* F, void* out, void* stream) {
   if (!p || !F || !out) return fail(MMX_ERR_ARG, "NULL plan or buffer");
   if (!p->kv_set) return fail(MMX_ERR_ARG, "k-vectors not set (mmx_plan_set_kvectors)");

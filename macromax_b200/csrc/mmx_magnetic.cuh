@@ -62,6 +62,51 @@ __global__ void k_curl_ft(const cpx<R>* __restrict__ F, cpx<R>* out, KGrid g, co
   }
 }
 
+// Longitudinal part k (k . F) / |k|^2 of a 3-component spectrum, or the transversal rest F minus it (backend/__init__.py:
+// 606-649: the zero frequency is longitudinal on the grid's axes, components without an axis have no longitudinal part).
+// One pass at the rate of memory: three words read and written per sample; a block takes rows of the contiguous axis, so
+// that only k of that axis changes within it.  150 x 128 x 110 complex128: 33 us, in place of 230 us of tensor operations.
+// May run in place (each sample is read before it is written, by the same thread).
+template <class R>
+__global__ void __launch_bounds__(256) k_project_ft(const cpx<R>* F, cpx<R>* out, KGrid g, const double* kv0,
+                                                    const double* kv1, const double* kv2, int transversal) {
+  const double* kv[3] = {kv0, kv1, kv2};
+  const int last = g.ndim - 1, n = g.dims[last];
+  const int64_t N = g.N, rows = N / n;
+  for (int64_t row = (int64_t)blockIdx.x * blockDim.y + threadIdx.y; row < rows; row += (int64_t)gridDim.x * blockDim.y) {
+    double k[3] = {0.0, 0.0, 0.0};
+    int64_t rest = row;
+    for (int a = last - 1; a >= 0; --a) {
+      const int64_t i = rest % g.dims[a];
+      rest /= g.dims[a];
+      k[a] = kv[a][i];
+    }
+    for (int i = threadIdx.x; i < n; i += blockDim.x) {
+      const int64_t v = row * n + i;
+      const double kl = kv[last][i];
+#pragma unroll
+      for (int a = 0; a < 3; ++a)
+        if (a == last) k[a] = kl;
+      cpx<R> f[3], pl[3];
+#pragma unroll
+      for (int c = 0; c < 3; ++c) f[c] = F[c * N + v];
+      if (v == 0) {
+#pragma unroll
+        for (int c = 0; c < 3; ++c) pl[c] = c <= last ? f[c] : mkc<R>((R)0, (R)0);
+      } else {
+        const double inv = 1.0 / (k[0] * k[0] + k[1] * k[1] + k[2] * k[2]);
+        cpx<R> proj = mkc<R>((R)0, (R)0);
+#pragma unroll
+        for (int c = 0; c < 3; ++c) proj += (R)k[c] * f[c];
+#pragma unroll
+        for (int c = 0; c < 3; ++c) pl[c] = (R)(k[c] * inv) * proj;
+      }
+#pragma unroll
+      for (int c = 0; c < 3; ++c) out[c * N + v] = transversal ? f[c] - pl[c] : pl[c];
+    }
+  }
+}
+
 // st: when not null, alpha is the right-hand side's current alpha (device-resident iteration) instead of (ar, ai)
 template <class R>
 __global__ void k_green_ft(cpx<R>* __restrict__ F, KGrid g, const R* kv0, const R* kv1, const R* kv2, R ar, R ai,

@@ -134,3 +134,28 @@ def test_fftn_matches_numpy(shape, dtype):
     nat.call('mmx_fftn', plan.handle, nat.device_ptr(yt), nat.device_ptr(yt), 2, 1, stream)  # in place, inverse
     assert np.linalg.norm(yt.cpu().numpy() - x) <= tol * np.linalg.norm(x)
     plan.close()
+
+
+@pytest.mark.parametrize('shape', [(7,), (300,), (13, 40), (64, 65), (5, 10, 20), (33, 4, 130)])
+@pytest.mark.parametrize('dtype', [np.complex64, np.complex128])
+def test_projections_match_tensor_expressions(shape, dtype):
+    import torch
+    from macromax_b200 import Grid
+    from macromax_b200.backend import BackEndB200
+    be = BackEndB200(3, Grid(shape=shape, step=125e-9), dtype)
+    rng = np.random.default_rng(2)
+    F = be.astype((rng.standard_normal((3, 1, *shape)) + 1j * rng.standard_normal((3, 1, *shape))).astype(dtype))
+    k = [np.asarray(x, dtype=np.float64) for x in be._grid.k]
+    k2 = sum(x ** 2 for x in k) + np.zeros(shape)
+    f = F.cpu().numpy().astype(np.complex128)[:, 0]
+    k2.flat[0] = 1.0
+    proj = sum(k[a] * f[a] for a in range(len(shape))) / k2
+    ref = np.zeros_like(f)
+    for a in range(len(shape)):
+        ref[a] = k[a] * proj
+        ref[a].flat[0] = f[a].flat[0]
+    tol = 4 * np.finfo(dtype).eps  # a few roundings per sample
+    conj = torch.conj(F)  # a lazily conjugated tensor
+    assert np.linalg.norm(be.longitudinal_projection_ft(F).cpu().numpy()[:, 0] - ref) <= tol * np.linalg.norm(f)
+    assert np.linalg.norm(be.transversal_projection_ft(F).cpu().numpy()[:, 0] - (f - ref)) <= tol * np.linalg.norm(f)
+    assert np.linalg.norm(be.transversal_projection_ft(conj).cpu().numpy()[:, 0] - np.conj(f - ref)) <= tol * np.linalg.norm(f)
