@@ -23,10 +23,14 @@ LIB_PATH = os.path.join(PKG, LIB_NAME)
 STAMP = LIB_PATH + '.srchash'
 
 OBJ_DIR = os.path.join(PKG, '_build')
-# compiled side by side and linked into one library; a translation unit whose sources did not change keeps its object
-SOURCES = ['mmx_capi.cu', 'mmx_loop.cu', 'mmx_loop_f64.cu', 'mmx_gen.cu', 'mmx_gen_f64.cu']
+# Translation units (source, definitions), compiled side by side and linked into one library; a unit whose sources did not
+# change keeps its object.  The longest first.
+UNITS = [('mmx_capi.cu', ())]
+UNITS += [('mmx_len.cu', (f'-DMMX_LEN_PART={part}', f'-DMMX_LEN_DOUBLE={double}')) for double in (1, 0)
+          for part in (0, 2, 1, 3)]
+UNITS += [(name, ()) for name in ('mmx_loop.cu', 'mmx_loop_f64.cu', 'mmx_gen.cu', 'mmx_gen_f64.cu')]
 NVCC_FLAGS = ['-gencode', 'arch=compute_100a,code=sm_100a', '-lineinfo', '-O3', '-std=c++17',
-              '-Xcompiler', '-fPIC', '-Xcompiler', '-O2']
+              '-Xcompiler', '-fPIC', '-Xcompiler', '-O2', '-Xfatbin', '-compress-all']
 
 
 def _nvcc() -> str:
@@ -55,10 +59,10 @@ def up_to_date() -> bool:
         return f.read().strip() == _source_hash()
 
 
-def _unit_hash(source: str) -> str:
+def _unit_hash(source: str, defs) -> str:
     """Of one translation unit: its source, the files of this tree that it includes, and the flags."""
     seen, todo = set(), [os.path.join(CSRC, source)]
-    h = hashlib.sha256(' '.join(NVCC_FLAGS).encode())
+    h = hashlib.sha256(' '.join([*NVCC_FLAGS, *defs]).encode())
     while todo:
         path = os.path.normpath(todo.pop())
         if path in seen or not os.path.exists(path):
@@ -71,15 +75,16 @@ def _unit_hash(source: str) -> str:
     return h.hexdigest()
 
 
-def _compile(source: str, force: bool, verbose: bool) -> str:
-    obj = os.path.join(OBJ_DIR, source + '.o')
+def _compile(unit, force: bool, verbose: bool) -> str:
+    source, defs = unit
+    obj = os.path.join(OBJ_DIR, source + ''.join(defs).replace('=', '') + '.o')
     stamp = obj + '.srchash'
-    digest = _unit_hash(source)
+    digest = _unit_hash(source, defs)
     if not force and os.path.exists(obj) and os.path.exists(stamp):
         with open(stamp) as f:
             if f.read().strip() == digest:
                 return obj
-    cmd = [_nvcc(), *NVCC_FLAGS, '-I', INCLUDE, '-c', '-o', obj + '.tmp', os.path.join(CSRC, source)]
+    cmd = [_nvcc(), *NVCC_FLAGS, *defs, '-I', INCLUDE, '-c', '-o', obj + '.tmp', os.path.join(CSRC, source)]
     if verbose:
         print(' '.join(cmd), flush=True)
     subprocess.run(cmd, check=True)
@@ -93,8 +98,8 @@ def build(force: bool = False, verbose: bool = False) -> str:
     if not force and up_to_date():
         return LIB_PATH
     os.makedirs(OBJ_DIR, exist_ok=True)
-    with ThreadPoolExecutor(max_workers=min(len(SOURCES), os.cpu_count() or 1)) as pool:
-        objs = list(pool.map(lambda src: _compile(src, force, verbose), SOURCES))
+    with ThreadPoolExecutor(max_workers=min(len(UNITS), os.cpu_count() or 1)) as pool:
+        objs = list(pool.map(lambda unit: _compile(unit, force, verbose), UNITS))
     tmp = LIB_PATH + '.tmp'
     cmd = [_nvcc(), *NVCC_FLAGS[:2], '-shared', '-o', tmp, *objs]
     if verbose:

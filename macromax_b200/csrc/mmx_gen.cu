@@ -103,36 +103,17 @@ GenTile gen_tile(GenKind kind, int n, int C, bool dbl, int64_t outer, int64_t in
   const bool rows = is_rows(kind);
   int maxT = 0;
   for (int s = 0; s < t.ax.nst; ++s) maxT = std::max(maxT, t.ax.T[s]);
-  // Strided: rows of 128 bytes (64 for the Green pass of a vector field, whose tile holds three components twice), down
-  // to one 32-byte sector while the launch has fewer than two tiles per SM.  Contiguous: rows for about 256 threads.
-  int P, floor = 1;
-  if (rows) {
-    P = 1;
-    while (2 * P * C * maxT <= 256 && P < 32) P *= 2;
-  } else {
-    P = (dbl ? 8 : 16) >> (kind == GEN_GREEN && C == 3 ? 1 : 0);
-    floor = dbl ? 2 : 4;
-  }
+  // narrower tiles while the launch has fewer than two per SM, down to one 32-byte sector of a row
+  int P = gen_width(kind, C, dbl, maxT);
+  const int full = P, floor = rows ? 1 : dbl ? 2 : 4;
   while (P > floor && ((pencils + P - 1) / P) * copies < 2 * (int64_t)sms) P /= 2;
   while (P > floor && tile_bytes(kind, t.ax, C, P, dbl) > 72 * 1024) P /= 2;
   if (tile_bytes(kind, t.ax, C, P, dbl) > kSmemCap) return t;
   t.lP = 0;
   while ((1 << t.lP) < P) ++t.lP;
-  // threads: the fewest thread-steps over the stages (a step costs its radix and a constant), more threads on a tie
-  const int unit = rows ? 32 : P;
-  const int per = rows ? C * P : (kind == GEN_GREEN ? C : 1);  // butterflies per T and unit column
-  long best = 0;
-  for (int thr = std::max(64, unit); thr <= 256; thr += unit) {
-    if (thr % 32) continue;
-    const int cols = rows ? thr : thr / P;
-    long cost = 0;
-    for (int s = 0; s < t.ax.nst; ++s) cost += (long)((per * t.ax.T[s] + cols - 1) / cols) * (t.ax.r[s] + 4);
-    cost *= thr;
-    if (!t.threads || cost <= best) {
-      best = cost;
-      t.threads = thr;
-    }
-  }
+  t.fixed = P == full && len_has(n) && pencils < (int64_t)1 << 31;
+  const int* r = t.ax.r;
+  t.threads = gen_threads(t.ax.nst, r[0], r[1], t.ax.nst > 2 ? r[2] : 1, t.ax.nst > 3 ? r[3] : 1, n, C, P, rows);
   t.smem = tile_bytes(kind, t.ax, C, P, dbl);
   t.tiles = (pencils + P - 1) / P;
   if (t.tiles > 0x7fffffff) t.threads = 0;
@@ -177,6 +158,15 @@ cudaError_t launch(const GenTile& t, const GenArgs<R>& a, int copies, bool pdl, 
 template <class R>
 cudaError_t gen_launch(GenKind kind, const GenTile& t, const IterArgs<R>& base, int C, int chi_kind, int dir, int batch,
                        const void* in, void* out, R scale, bool pdl, cudaStream_t s) {
+  if (t.fixed && chi_kind != MMX_CHI_MAT3) {
+    static_assert(kLenParts == 4, "one case per part");
+    switch (t.ax.n % kLenParts) {
+      case 0: return len_launch<R, 0>(kind, t, base, C, dir, batch, in, out, scale, pdl, s);
+      case 1: return len_launch<R, 1>(kind, t, base, C, dir, batch, in, out, scale, pdl, s);
+      case 2: return len_launch<R, 2>(kind, t, base, C, dir, batch, in, out, scale, pdl, s);
+      default: return len_launch<R, 3>(kind, t, base, C, dir, batch, in, out, scale, pdl, s);
+    }
+  }
   GenArgs<R> a;
   static_cast<IterArgs<R>&>(a) = base;
   a.g = t.ax;

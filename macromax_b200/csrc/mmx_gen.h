@@ -26,8 +26,38 @@ enum GenKind : int {
   GEN_EPI3
 };
 
+// Pencils (rows) per tile, before a launch of few tiles narrows them.  Strided: rows of 128 bytes (64 for the Green pass of
+// a vector field, whose tile holds three components twice).  Contiguous: rows for about 256 threads (maxT: the most
+// butterflies per row of a stage).
+constexpr int gen_width(GenKind kind, int C, bool dbl, int maxT) {
+  if (kind == GEN_STRIDED || kind == GEN_GREEN) return (dbl ? 8 : 16) >> (kind == GEN_GREEN && C == 3 ? 1 : 0);
+  int P = 1;
+  while (2 * P * C * maxT <= 256 && P < 32) P *= 2;
+  return P;
+}
+// Threads of a tile: the fewest thread-steps over its stages (a step costs its radix and a constant), more threads on a
+// tie.  C: components in the tile.
+constexpr int gen_threads(int nst, int r0, int r1, int r2, int r3, int n, int C, int P, bool rows) {
+  const int r[4] = {r0, r1, r2, r3};
+  int threads = 0;
+  long best = 0;
+  for (int thr = 64; thr <= 256; thr += 32) {
+    if (!rows && thr % P) continue;
+    const int cols = rows ? thr : thr / P, per = rows ? C * P : C;
+    long cost = 0;
+    for (int s = 0; s < nst; ++s) cost += (long)((per * (n / r[s]) + cols - 1) / cols) * (r[s] + 4);
+    cost *= thr;
+    if (!threads || cost <= best) {
+      best = cost;
+      threads = thr;
+    }
+  }
+  return threads;
+}
+
 struct GenTile {
   GenAxis ax;
+  bool fixed = false;  // the length has a kernel of its own (mmx_len.cuh) and the tile is the one it is compiled for
   int lP = 0;       // log2 of the pencils (rows) per tile
   int threads = 0;  // 0: no such pass (the axis has no plan, or its tile does not fit)
   size_t smem = 0;
@@ -41,9 +71,24 @@ bool gen_small_plan(int n, GenAxis* ax);
 // number of independent such passes in one launch (right-hand sides, or components of them).
 GenTile gen_tile(GenKind kind, int n, int C, bool dbl, int64_t outer, int64_t inner, int64_t copies, int sms);
 
+// Lengths with kernels of their own: 32 .. 192, the product of two radices up to 16.
+constexpr int kLenFirst = 32, kLenLast = 192;
+constexpr bool len_has(int n) {
+  if (n < kLenFirst || n > kLenLast) return false;
+  for (int a = 2; a <= 16; ++a)
+    if (n % a == 0 && n / a <= 16) return true;
+  return false;
+}
+
 // Launch one pass.  a: the iteration arguments (outer, inner, T, ... set by the caller; st may be null for the plain
 // transforms).  in / out / scale: the plain transforms' buffers and factor; C: the field's components; fields: the
 // launch's second dimension for the plain transforms; dir: -1 forward, +1 inverse.  pdl: programmatic dependent launch.
 template <class R>
 cudaError_t gen_launch(GenKind kind, const GenTile& t, const IterArgs<R>& a, int C, int chi_kind, int dir, int batch,
                        const void* in, void* out, R scale, bool pdl, cudaStream_t s);
+
+// The same for a tile with `fixed` set, by length; part: lengths with n % kLenParts == part are compiled there.
+constexpr int kLenParts = 4;
+template <class R, int PART>
+cudaError_t len_launch(GenKind kind, const GenTile& t, const IterArgs<R>& a, int C, int dir, int batch, const void* in,
+                       void* out, R scale, bool pdl, cudaStream_t s);

@@ -59,6 +59,22 @@ def test_iteration_matches_generic_and_oracle(shape, components, medium, dtype, 
     assert fast.residue == pytest.approx(gen.residue, rel=10 * tol)
 
 
+# enough tiles for the kernels compiled for their length on every axis: the smallest and the largest, odd ones, radix 16
+@pytest.mark.parametrize('shape,components,medium', [((35, 72, 80), 3, 'scalar'), ((143, 66, 75), 1, 'scalar'),
+                                                     ((32, 182, 77), 3, 'symmetric'), ((192, 70, 72), 1, 'scalar'),
+                                                     ((60, 110, 169), 3, 'scalar'), ((112, 108, 45), 3, 'symmetric'),
+                                                     ((64, 96, 90), 3, 'general')])
+@pytest.mark.parametrize('dtype', [np.complex64, np.complex128])
+def test_lengths_with_own_kernels_match_generic(shape, components, medium, dtype):
+    wl = _problem(shape, components, medium)
+    fast, gen = _solution(wl, dtype), _solution(wl, dtype, generic=True)
+    for s in (fast, gen):
+        s.solve(None, rtol=0, maxiter=6)
+    tol = 1e-5 if dtype == np.complex64 else 1e-12
+    assert rel(fast.E, gen.E) < tol
+    assert fast.residue == pytest.approx(gen.residue, rel=10 * tol)
+
+
 @pytest.mark.parametrize('shape,components', [((1000,), 1), ((77,), 3), ((4,), 1), ((2160,), 1), ((825,), 3)])
 @pytest.mark.parametrize('dtype', [np.complex64, np.complex128])
 def test_line_matches_generic_and_oracle(shape, components, dtype):
@@ -115,7 +131,8 @@ def test_batch_members_match_single_solves(shape, components, batch):
     bs.close()
 
 
-@pytest.mark.parametrize('shape', [(22, 26), (1500, 9), (4, 1100), (150, 128, 110), (39, 35, 143), (2048, 6), (13, 13)])
+@pytest.mark.parametrize('shape', [(22, 26), (1500, 9), (4, 1100), (150, 128, 110), (39, 35, 143), (2048, 6), (13, 13),
+                                   (60, 77, 96), (192, 100, 33)])
 @pytest.mark.parametrize('dtype', [np.complex64, np.complex128])
 def test_fftn_matches_numpy(shape, dtype):
     import torch
