@@ -981,10 +981,10 @@ bool epro_runs(const mmx_plan* p, int chi_kind) {
 // The configuration under which a chunk of iterations runs in one launch, or null.  It does in the default variant where
 // the CTAs can keep the rows of the grid in shared memory (loop_config; up to about 900 000 scalar complex64 samples),
 // except on complex64 grids whose passes are all specialised for their length: those keep the rounding that their other
-// variants and their branch of an uneven batch have, and gain least.  us per iteration, one launch against passes: complex64 300 x 420 15.8 / 30.0, 8 sources
-// on 200 x 180 20.2 / 29.6, 48 x 42 x 44 17.7 / 30.6 (vector: 25.6 / 33.5); specialised: 64^2 8.6 / 13.1, 256^2 12.7 / 18.0,
-// 512^2 22.4 / 24.0, 64^3 20.0 / 18.8; complex128 64^2 8.5 / 20.8, 256^2 11.2 / 32.9, 512^2 23.1 / 29.6, 64^3 27.0 / 34.8;
-// 1000 samples in 1D 7.9 / 20.0 (complex128 8.0 / 24.2).
+// variants and their branch of an uneven batch have, and gain least.  us per iteration, one launch against passes:
+// complex64 300 x 420 14.3 / 30.0, 8 sources on 200 x 180 19.0 / 29.6, 48 x 42 x 44 18.5 / 30.6 (vector: 23.5 / 33.5);
+// specialised: 64^2 9.3 / 13.1, 256^2 11.9 / 18.0, 512^2 22.4 / 24.0, 64^3 20.0 / 18.8; complex128 64^2 8.7 / 20.8, 256^2
+// 11.7 / 32.9, 512^2 23.1 / 29.6, 64^3 27.0 / 34.8; 1000 samples in 1D 6.2 / 20.0 (complex128 6.6 / 24.2).
 const LoopCfg* loop_runs(mmx_plan* p, int chi_kind) {
   if (p->force_generic || p->no_reg || p->pipe || p->plane || p->epro || p->tma || p->runtime_radix || p->passes_only ||
       p->compare_green || p->l2_persist)

@@ -81,15 +81,25 @@ size_t tile_bytes(GenKind kind, const GenAxis& ax, int C, int P, bool dbl) {
 }  // namespace
 
 bool gen_small_plan(int n, GenAxis* ax) {
-  int r[MMX_GEN_STAGES], nst = 0, m = n;
-  for (int f : {13, 11, 7, 5, 4, 3, 2})
-    while (m % f == 0 && m > 1) {
-      if (nst == MMX_GEN_STAGES) return false;
-      r[nst++] = f;
+  int r[MMX_GEN_STAGES], primes = 0, m = n;
+  for (int f : {13, 11})
+    while (m % f == 0) {
+      if (primes == MMX_GEN_STAGES) return false;
+      r[primes++] = f;
       m /= f;
     }
-  if (n == 4) nst = 2, r[0] = r[1] = 2;
-  if (m != 1 || nst < 2) return false;
+  int nst = primes;
+  if (m > 1) {
+    int sum = 0;
+    bool found = false;
+    for (int stages = primes ? 1 : 2; !found && primes + stages <= MMX_GEN_STAGES; ++stages)
+      if (best_radices(m, stages, 10, r + primes, &sum)) {
+        found = true;
+        nst = primes + stages;
+      }
+    if (!found) return false;
+  }
+  if (nst < 2) return false;
   fill_axis(n, nst, r, ax);
   return true;
 }

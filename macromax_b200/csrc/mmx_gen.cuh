@@ -81,14 +81,18 @@ struct WideRadices {  // 2 .. 16: few stages, for passes that are bound by traff
     }
   }
 };
-struct SmallRadices {  // 4, 5, 3, 2 and the other primes: short butterflies on many threads, for launches bound by latency
+struct SmallRadices {  // up to 10 and the primes: shorter butterflies on more threads, for launches bound by latency
   template <class F> static __device__ __forceinline__ void run(int r, F&& f) {
     switch (r) {
       case 2: f(std::integral_constant<int, 2>{}); break;
       case 3: f(std::integral_constant<int, 3>{}); break;
       case 4: f(std::integral_constant<int, 4>{}); break;
       case 5: f(std::integral_constant<int, 5>{}); break;
+      case 6: f(std::integral_constant<int, 6>{}); break;
       case 7: f(std::integral_constant<int, 7>{}); break;
+      case 8: f(std::integral_constant<int, 8>{}); break;
+      case 9: f(std::integral_constant<int, 9>{}); break;
+      case 10: f(std::integral_constant<int, 10>{}); break;
       case 11: f(std::integral_constant<int, 11>{}); break;
       default: f(std::integral_constant<int, 13>{}); break;
     }

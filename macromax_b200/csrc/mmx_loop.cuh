@@ -9,8 +9,7 @@
 //   in 3D the middle axis forward before and inverse after axis 0
 //
 // What bounds it is latency: a thread's instructions from one barrier to the next, and the trips to L2.  So the stages
-// have radices 4, 5, 3, 2 (a radix-16 butterfly is one thread's work for a thousand cycles, four times that of two
-// radix-4 stages on four times the threads), and whatever a CTA meets again stays in shared memory: the fields, chi and
+// have radices up to 10 (a radix-16 butterfly is one thread's work for a thousand cycles), and whatever a CTA meets again stays in shared memory: the fields, chi and
 // sources of its rows (loaded once, the fields written back at the end), the twiddles, the k tables, the states of the
 // right-hand sides and the coefficients that follow from them.  Only the work buffer crosses L2.
 //
