@@ -143,7 +143,8 @@ def check(rc: int):
 
 def check_stalled(states):
     """Raise when a launch whose blocks wait for one another gave up (MMX_STATUS_STALLED): its fields are not valid."""
-    if np.any(np.asarray(states['status']) & MMX_STATUS_STALLED):
+    status = states['status']
+    if (int(status) if status.ndim == 0 else int(np.bitwise_or.reduce(status))) & MMX_STATUS_STALLED:
         raise NativeError('the blocks of an iteration launch did not run together; set another variant '
                           '(MMX_VARIANT_PASSES) for this plan')
 

@@ -54,6 +54,21 @@ def pack_symmetric(chi: torch.Tensor) -> tuple[torch.Tensor, int]:
     return chi, nat.MMX_CHI_MAT3
 
 
+_thread = threading.local()
+_STAGING_BYTES = 1 << 16
+
+
+def _staging(nbytes: int):
+    """The first ``nbytes`` of this thread's pinned buffer for reading states (64 KiB, one per thread for the life of the
+    thread; None for more)."""
+    if nbytes > _STAGING_BYTES:
+        return None
+    buf = getattr(_thread, 'staging', None)
+    if buf is None:
+        buf = _thread.staging = torch.empty(_STAGING_BYTES, dtype=torch.uint8, pin_memory=True)
+    return buf[:nbytes]
+
+
 class IterationEngine:
     def __init__(self, shape, ncomp: int, batch: int, dtype, ks, chi0: np.ndarray, alpha0: complex,
                  device=None):
@@ -74,8 +89,6 @@ class IterationEngine:
             self.fields = torch.zeros((2, self.batch, self.ncomp, self.N), dtype=self.torch_dtype, device=self.device)
             self.sources = torch.zeros((self.batch, self.ncomp, self.N), dtype=self.torch_dtype, device=self.device)
             self.state = torch.zeros((self.batch, nat.STATE_DTYPE.itemsize), dtype=torch.uint8, device=self.device)
-        self._state_host = torch.empty(self.state.shape, dtype=torch.uint8, pin_memory=True)
-        self._state_lock = threading.Lock()
         self._launches = 0  # iteration calls so far: with the state tensor's version, what a copy of the state is of
         self.set_chi(chi0, alpha0)
         st = np.zeros(self.batch, dtype=nat.STATE_DTYPE)
@@ -152,10 +165,12 @@ class IterationEngine:
 
     # -- state ------------------------------------------------------------------------------------------------------
     def read_state(self) -> np.ndarray:
-        with self._state_lock:  # one staging buffer
-            self._state_host.copy_(self.state, non_blocking=True)
-            torch.cuda.current_stream(self.device).synchronize()
-            return self._state_host.numpy().view(nat.STATE_DTYPE).reshape(self.batch).copy()
+        host = _staging(self.state.numel())
+        if host is None:
+            return self.state.cpu().numpy().view(nat.STATE_DTYPE).reshape(self.batch).copy()
+        host.copy_(self.state.view(-1), non_blocking=True)
+        torch.cuda.current_stream(self.device).synchronize()
+        return host.numpy().view(nat.STATE_DTYPE).copy()
 
     def state_key(self):
         """Changes with every iteration call and with every write to the state tensor."""
