@@ -1276,9 +1276,12 @@ int mmx_plan_create(int ndim, const int64_t* shape, int ncomp, int batch, int pr
     p->kv_off[i] = kv_total;
     kv_total += n;
   }
-  cudaError_t e = cudaMalloc(&p->kv_dev, (wb / 2) * (size_t)kv_total);
-  if (e == cudaSuccess) e = cudaMemset(p->kv_dev, 0, (wb / 2) * (size_t)kv_total);
-  if (e == cudaSuccess && precision == MMX_C64) e = cudaMalloc(&p->kvd_dev, sizeof(double) * (size_t)kv_total);
+  // the k tables in the plan's precision, and behind them (complex64) the same in FP64
+  const size_t kv_bytes = ((wb / 2) * (size_t)kv_total + 15) & ~(size_t)15;
+  const size_t kv_all = kv_bytes + (precision == MMX_C64 ? sizeof(double) * (size_t)kv_total : 0);
+  cudaError_t e = cudaMalloc(&p->kv_dev, kv_all);
+  if (e == cudaSuccess) e = cudaMemset(p->kv_dev, 0, kv_all);
+  if (e == cudaSuccess && precision == MMX_C64) p->kvd_dev = (double*)((unsigned char*)p->kv_dev + kv_bytes);
   if (e == cudaSuccess) e = cudaMalloc(&p->work, wb * (size_t)batch * ncomp * p->N);
   if (e != cudaSuccess) {
     mmx_plan_destroy(p);
@@ -1344,7 +1347,6 @@ int mmx_plan_destroy(mmx_plan* p) {
   for (int i = 0; i < 3; ++i)
     if (p->tw_dev[i]) cudaFree(p->tw_dev[i]);
   if (p->kv_dev) cudaFree(p->kv_dev);
-  if (p->kvd_dev) cudaFree(p->kvd_dev);
   if (p->work) cudaFree(p->work);
   if (p->partials) cudaFree(p->partials);
   if (p->done) cudaFree(p->done);

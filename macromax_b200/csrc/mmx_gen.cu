@@ -123,7 +123,8 @@ GenTile gen_tile(GenKind kind, int n, int C, bool dbl, int64_t outer, int64_t in
   while ((1 << t.lP) < P) ++t.lP;
   t.fixed = P == full && len_has(n) && pencils < (int64_t)1 << 31;
   const int* r = t.ax.r;
-  t.threads = gen_threads(t.ax.nst, r[0], r[1], t.ax.nst > 2 ? r[2] : 1, t.ax.nst > 3 ? r[3] : 1, n, C, P, rows);
+  t.threads = gen_threads(t.ax.nst, r[0], r[1], t.ax.nst > 2 ? r[2] : 1, t.ax.nst > 3 ? r[3] : 1, n, C, P, rows,
+                          (long)tile_bytes(kind, t.ax, C, P, dbl));
   t.smem = tile_bytes(kind, t.ax, C, P, dbl);
   t.tiles = (pencils + P - 1) / P;
   if (t.tiles > 0x7fffffff) t.threads = 0;

@@ -35,9 +35,10 @@ constexpr int gen_width(GenKind kind, int C, bool dbl, int maxT) {
   while (2 * P * C * maxT <= 256 && P < 32) P *= 2;
   return P;
 }
-// Threads of a tile: the fewest thread-steps over its stages (a step costs its radix and a constant), more threads on a
-// tie.  C: components in the tile.
-constexpr int gen_threads(int nst, int r0, int r1, int r2, int r3, int n, int C, int P, bool rows) {
+// Threads of a tile: the fewest thread-steps over its stages (a step costs its radix and a constant), where the tiles that
+// fit an SM at once (smem bytes each, at most 1024 threads) bring it 1024 threads or nearly; more threads on a tie.
+// C: components in the tile.  The 126-sample strided pass took 16.5 us with 64 threads, which is 24 warps on an SM.
+constexpr int gen_threads(int nst, int r0, int r1, int r2, int r3, int n, int C, int P, bool rows, long smem) {
   const int r[4] = {r0, r1, r2, r3};
   int threads = 0;
   long best = 0;
@@ -46,7 +47,9 @@ constexpr int gen_threads(int nst, int r0, int r1, int r2, int r3, int n, int C,
     const int cols = rows ? thr : thr / P, per = rows ? C * P : C;
     long cost = 0;
     for (int s = 0; s < nst; ++s) cost += (long)((per * (n / r[s]) + cols - 1) / cols) * (r[s] + 4);
-    cost *= thr;
+    const long by_smem = 227 * 1024 / (smem + 1024), by_regs = 1024 / thr;
+    const long resident = (by_smem < by_regs ? by_smem : by_regs) * thr;
+    cost = cost * thr * 1024 / (resident < 1 ? 1 : resident);
     if (!threads || cost <= best) {
       best = cost;
       threads = thr;

@@ -41,9 +41,9 @@ template <class R> struct LenArgs : IterArgs<R> {
 template <class R, int N> struct LenStrided {
   using L = LenPlan<N, true>;
   static constexpr int P = gen_width(GEN_STRIDED, 1, sizeof(R) == 8, 0);
-  static constexpr int THREADS = gen_threads(2, L::R0, L::R1, 0, 0, N, 1, P, false);
-  static constexpr int BLOCKS = len_blocks(THREADS, kLenRegs<R, L::R0>);
   static constexpr size_t SMEM = N * sizeof(gtw<R>) + (size_t)N * P * sizeof(cpx<R>);
+  static constexpr int THREADS = gen_threads(2, L::R0, L::R1, 0, 0, N, 1, P, false, SMEM);
+  static constexpr int BLOCKS = len_blocks(THREADS, kLenRegs<R, L::R0>);
 };
 template <class R, int DIR, int N>
 __global__ void __launch_bounds__(LenStrided<R, N>::THREADS, (LenStrided<R, N>::BLOCKS))
@@ -102,10 +102,10 @@ __global__ void __launch_bounds__(LenStrided<R, N>::THREADS, (LenStrided<R, N>::
 template <class R, int C, int N> struct LenGreen {
   using L = LenPlan<N, true>;
   static constexpr int P = gen_width(GEN_GREEN, C, sizeof(R) == 8, 0);
-  static constexpr int THREADS = gen_threads(2, L::R0, L::R1, 0, 0, N, C, P, false);
-  static constexpr int BLOCKS = len_blocks(THREADS, kLenRegs<R, L::R0>);
   static constexpr size_t SMEM =
       N * sizeof(gtw<R>) + (C == 3 ? 2 : 1) * (size_t)C * N * P * sizeof(cpx<R>) + N * sizeof(double);
+  static constexpr int THREADS = gen_threads(2, L::R0, L::R1, 0, 0, N, C, P, false, SMEM);
+  static constexpr int BLOCKS = len_blocks(THREADS, kLenRegs<R, L::R0>);
 };
 template <class R, int C, int N>
 __global__ void __launch_bounds__(LenGreen<R, C, N>::THREADS, (LenGreen<R, C, N>::BLOCKS))
@@ -264,10 +264,12 @@ template <class R, int KIND, int C, int N> struct LenRows {
   using L = LenPlan<N, KIND == GEN_EPI>;
   static constexpr int P = gen_width((GenKind)KIND, C, sizeof(R) == 8, L::T0 > L::T1 ? L::T0 : L::T1);
   static constexpr int ROWS = C * P;
-  static constexpr int THREADS = gen_threads(2, L::R0, L::R1, 0, 0, N, C, P, true);
-  static constexpr int BLOCKS = len_blocks(THREADS, kLenRegs<R, (L::R0 > L::R1 ? L::R0 : L::R1)>);
   static constexpr int W0 = L::T0 * L::G;  // words of a row after the first stage
   static constexpr size_t SMEM = N * sizeof(gtw<R>) + (size_t)ROWS * (W0 + (k3 ? N : 0)) * sizeof(cpx<R>);
+  static constexpr int THREADS = gen_threads(2, L::R0, L::R1, 0, 0, N, C, P, true, SMEM);
+  // the epilogue holds E and chi of half a butterfly beside it
+  static constexpr int REGS = kLenRegs<R, (L::R0 > L::R1 ? L::R0 : L::R1)>;
+  static constexpr int BLOCKS = len_blocks(THREADS, KIND == GEN_EPI && REGS < 80 ? 80 : REGS);
 };
 template <class R, int KIND, int C, int DIR, int N>
 __global__ void __launch_bounds__(LenRows<R, KIND, C, N>::THREADS, (LenRows<R, KIND, C, N>::BLOCKS))
@@ -282,7 +284,11 @@ __global__ void __launch_bounds__(LenRows<R, KIND, C, N>::THREADS, (LenRows<R, K
   cpx<R>* sm = reinterpret_cast<cpx<R>*>(tw + N);  // [row][T0 groups of R0 words at pitch G]
   cpx<R>* sn = sm + ROWS * K::W0;                  // 3x3: [row][N]
   const int tid = threadIdx.x;
-  for (int t = tid; t < N; t += THREADS) tw[t] = GenTw<R>::load(a.ax, t);
+  // the factors of butterfly i at [q - 1][i]: neighbouring threads read neighbouring words
+  for (int t = tid; t < (L::R1 - 1) * L::T1; t += THREADS) {
+    const int q = t / L::T1;
+    tw[t] = GenTw<R>::load(a.ax, (q + 1) * (t - q * L::T1));
+  }
   const int b = blockIdx.y;
   const int64_t row0 = (int64_t)blockIdx.x * P;
   const int left = a.outer - row0 < P ? (int)(a.outer - row0) : P;
@@ -358,24 +364,29 @@ __global__ void __launch_bounds__(LenRows<R, KIND, C, N>::THREADS, (LenRows<R, K
     const int64_t off = c * NV + row * N + i;
     cpx<R> u[L::R1];
     const cpx<R>* s = sm + r * K::W0 + i;
+    // E and chi of CH samples are in flight at a time, the first ones while the butterfly is computed
+    constexpr int CH = !kEpi ? 1 : L::R1 <= 6 ? L::R1 : (L::R1 + 1) / 2;
+    cpx<R> ev[CH], xv[CH];
+    const cpx<R>*eS = E + off, *xS = X + row * N + i;
+    auto fetch = [&](int q0) {
+#pragma unroll
+      for (int q = 0; q < CH; ++q)
+        if (q0 + q < L::R1) {
+          ev[q] = eS[(q0 + q) * L::T1];
+          xv[q] = xS[(q0 + q) * L::T1];
+        }
+    };
+    if constexpr (kEpi) fetch(0);
 #pragma unroll
     for (int q = 0; q < L::R1; ++q) u[q] = s[q * L::G];
 #pragma unroll
-    for (int q = 1; q < L::R1; ++q) u[q] = GenTw<R>::template mul<DIR>(u[q], tw[q * i]);
+    for (int q = 1; q < L::R1; ++q) u[q] = GenTw<R>::template mul<DIR>(u[q], tw[(q - 1) * L::T1 + i]);
     gdft<R, L::R1, DIR>(u);
     if constexpr (kEpi) {
-      const cpx<R>*eS = E + off, *xS = X + row * N + i;
       cpx<R>* eO = En + off;
-      constexpr int CH = L::R1 <= 8 ? L::R1 : (L::R1 + 1) / 2;  // samples whose E and chi are in flight
 #pragma unroll
       for (int q0 = 0; q0 < L::R1; q0 += CH) {
-        cpx<R> ev[CH], xv[CH];
-#pragma unroll
-        for (int q = 0; q < CH; ++q)
-          if (q0 + q < L::R1) {
-            ev[q] = eS[(q0 + q) * L::T1];
-            xv[q] = xS[(q0 + q) * L::T1];
-          }
+        if (q0 > 0) fetch(q0);
 #pragma unroll
         for (int q = 0; q < CH; ++q)
           if (q0 + q < L::R1) {
