@@ -185,6 +185,9 @@ int mmx_adjoint_grad(const void* E, const void* nu, void* grad, int64_t batch, i
 int mmx_pointwise_mul(const void* A, int ra, int ca, const void* B, int cb, int b_broadcast, void* out,
                       int64_t nvox, int precision, void* stream);
 
+/* Copy `bytes` from the device to the host (pinned memory: at once) and wait for the stream: the states after a chunk. */
+int mmx_read_back(void* host, const void* device, int64_t bytes, void* stream);
+
 /* 1 when a chunk of iterations of this plan runs in one launch that ends when no right-hand side is active any more, so
  * that a chunk longer than the solve costs nothing; 0 when every iteration is launched (and may leave at once). */
 int mmx_plan_chunk_ends(mmx_plan* plan, int chi_kind);

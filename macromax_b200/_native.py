@@ -121,6 +121,7 @@ def load(path: str | None = None):
         'mmx_mode_scatter': (i32, [vp, vp, i64, i64, i64, i32, vp, i32, vp]),
         'mmx_mode_gather': (i32, [vp, vp, i64, i64, i64, i32, vp, i32, vp]),
         'mmx_plan_set_variant': (i32, [vp, ctypes.c_uint]),
+        'mmx_read_back': (i32, [vp, vp, i64, vp]),
         'mmx_plan_chunk_ends': (i32, [vp, i32]),
         'mmx_plan_get_variant': (ctypes.c_uint, [vp]),
         'mmx_iterate_multi': (i32, [i32, ctypes.POINTER(vp), ctypes.POINTER(vp), ctypes.POINTER(vp),

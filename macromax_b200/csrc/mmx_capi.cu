@@ -1677,6 +1677,13 @@ extern "C" int mmx_plan_set_variant(mmx_plan* p, unsigned flags) {
   return MMX_OK;
 }
 
+extern "C" int mmx_read_back(void* host, const void* device, int64_t bytes, void* stream) {
+  if (!host || !device || bytes < 0) return fail(MMX_ERR_ARG, "NULL buffer or negative size");
+  MMX_CUDA(cudaMemcpyAsync(host, device, (size_t)bytes, cudaMemcpyDeviceToHost, (cudaStream_t)stream));
+  MMX_CUDA(cudaStreamSynchronize((cudaStream_t)stream));
+  return MMX_OK;
+}
+
 extern "C" int mmx_plan_chunk_ends(mmx_plan* p, int chi_kind) {
   if (!p || (chi_kind != MMX_CHI_SCALAR && chi_kind != MMX_CHI_MAT3 && chi_kind != MMX_CHI_SYM6)) return 0;
   return loop_runs(p, chi_kind) != nullptr;

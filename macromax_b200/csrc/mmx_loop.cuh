@@ -436,6 +436,11 @@ __global__ void __launch_bounds__(kLoopThreads, sizeof(R) == 4 ? 2 : 1) k_loop(c
     } else if (pending && pass == after_rows) {
       decide();
     }
+    if (finished) {  // nothing follows the last decision, which every CTA has taken for itself
+      __syncthreads();
+      cur ^= 1;
+      break;
+    }
     if (!(ok = barrier())) break;
     if (pass == ROWS) {
       pending = (mode & LOOP_EPI) != 0;
@@ -446,7 +451,7 @@ __global__ void __launch_bounds__(kLoopThreads, sizeof(R) == 4 ? 2 : 1) k_loop(c
       if (pending) {
         pending = false;
         cur ^= 1;
-        if (finished || !flags[0]) break;
+        if (!flags[0]) break;
         if (flags[1]) {  // the rejected right-hand sides' input again, from the old field
           redo = true;
           mode = LOOP_PRO;

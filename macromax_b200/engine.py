@@ -65,7 +65,8 @@ def _staging(nbytes: int):
         return None
     buf = getattr(_thread, 'staging', None)
     if buf is None:
-        buf = _thread.staging = torch.empty(_STAGING_BYTES, dtype=torch.uint8, pin_memory=True)
+        _thread.pinned = torch.empty(_STAGING_BYTES, dtype=torch.uint8, pin_memory=True)
+        buf = _thread.staging = _thread.pinned.numpy()
     return buf[:nbytes]
 
 
@@ -166,11 +167,11 @@ class IterationEngine:
     # -- state ------------------------------------------------------------------------------------------------------
     def read_state(self) -> np.ndarray:
         host = _staging(self.state.numel())
-        if host is None:
+        if host is None or torch.cuda.current_device() != self.state.device.index:
             return self.state.cpu().numpy().view(nat.STATE_DTYPE).reshape(self.batch).copy()
-        host.copy_(self.state.view(-1), non_blocking=True)
-        torch.cuda.current_stream(self.device).synchronize()
-        return host.numpy().view(nat.STATE_DTYPE).copy()
+        nat.call('mmx_read_back', host.ctypes.data, self.state.data_ptr(), host.nbytes,
+                 torch.cuda.current_stream(self.device).cuda_stream)
+        return host.view(nat.STATE_DTYPE).copy()
 
     def state_key(self):
         """Changes with every iteration call and with every write to the state tensor."""
@@ -230,8 +231,11 @@ class IterationEngine:
             fn = 'mmx_iterate_graph_continue' if cont else 'mmx_iterate_graph'
         else:
             fn = 'mmx_iterate'
-        nat.call(fn, self.plan.handle, _ptr(self.fields[0]), _ptr(self.fields[1]), _ptr(self.chi),
-                 self.chi_kind, _ptr(self.sources), _ptr(self.state), int(niter), _stream_ptr(stream))
+        E = _ptr(self.fields)  # the two buffers, one behind the other
+        half = self.fields.numel() // 2 * self.fields.element_size()
+        s = stream if stream is not None else torch.cuda.current_stream()
+        nat.call(fn, self.plan.handle, E, E.value + half, _ptr(self.chi), self.chi_kind, _ptr(self.sources),
+                 _ptr(self.state), int(niter), s.cuda_stream)
 
     def prepare_graph(self, niter: int):
         """Capture the graph of an ``niter``-iteration chunk now (so that a later timed chunk does not)."""
