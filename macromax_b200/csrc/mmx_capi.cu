@@ -132,7 +132,7 @@ struct mmx_plan {
   int prec = MMX_C64;
   int64_t N = 1;
   FFTAxis ax[3];           // radix plans; tw points at device twiddles of the plan precision
-  void* tw_dev[3] = {nullptr, nullptr, nullptr};
+  void* small = nullptr;   // the allocation that holds the tables, the counters and the partial sums
   void* kv_dev = nullptr;  // k tables, plan precision, concatenated
   double* kvd_dev = nullptr;  // the same in FP64 (complex64 plans; complex128 plans use kv_dev)
   int kv_off[3] = {0, 0, 0};
@@ -1241,52 +1241,64 @@ int mmx_plan_create(int ndim, const int64_t* shape, int ncomp, int batch, int pr
   }
   for (int i = ndim; i < 3; ++i) p->shape[i] = 1;
   const size_t wb = word_bytes(precision);
-  // twiddles exp(-2 pi i t / n), computed in FP64
+  // One allocation and one copy for everything but the work buffer (an allocation and its release take a fraction of a
+  // millisecond each, and a plan of a small problem is made for every solve of an optimisation): the twiddle tables, the k
+  // tables in the plan's precision and (complex64) in FP64, the counters, and the partial sums behind the copied part.
+  auto up = [](size_t x) { return (x + 255) & ~(size_t)255; };
+  const bool single = precision == MMX_C64;
+  size_t off = 0, tw_off[3] = {0, 0, 0};
   int kv_total = 0;
   for (int i = 0; i < ndim; ++i) {
+    tw_off[i] = off;
+    off = up(off + (single ? 2 : 1) * wb * (size_t)shape[i]);
+    p->kv_off[i] = kv_total;
+    kv_total += (int)shape[i];
+  }
+  const size_t kv_off = off;
+  off = up(off + (wb / 2) * (size_t)kv_total);
+  const size_t kvd_off = off;
+  if (single) off = up(off + sizeof(double) * (size_t)kv_total);
+  const size_t done_off = off;
+  off = up(off + sizeof(unsigned int) * ((size_t)batch + 2));
+  int64_t maxt = 2048;  // enough partial sums for any tile width (at most one tile per pencil)
+  for (int i = 0; i < ndim; ++i) maxt = std::max<int64_t>(maxt, p->N / shape[i]);
+  p->partials_len = (int64_t)batch * maxt * 2;
+  std::vector<unsigned char> image(off, 0);
+  for (int i = 0; i < ndim; ++i) {  // exp(-2 pi i t / n), computed in FP64
     const int n = (int)shape[i];
-    std::vector<double> twd(2 * (size_t)n);
+    double* td = (double*)(image.data() + tw_off[i]);
+    float* tf = (float*)td;  // complex64: the table, and behind it what rounding to float took from it
     for (int t = 0; t < n; ++t) {
       const double ang = -2.0 * M_PI * (double)t / (double)n;
-      twd[2 * t] = std::cos(ang);
-      twd[2 * t + 1] = std::sin(ang);
-    }
-    // complex64: the table, and behind it what rounding to float took from it
-    cudaError_t e = cudaMalloc(&p->tw_dev[i], (precision == MMX_C64 ? 2 : 1) * wb * n);
-    if (e != cudaSuccess) {
-      mmx_plan_destroy(p);
-      return cuda_fail(e, "cudaMalloc(twiddles)");
-    }
-    if (precision == MMX_C128) {
-      e = cudaMemcpy(p->tw_dev[i], twd.data(), wb * n, cudaMemcpyHostToDevice);
-    } else {
-      std::vector<float> twf(4 * (size_t)n);
-      for (size_t k = 0; k < twd.size(); ++k) {
-        twf[k] = (float)twd[k];
-        twf[twd.size() + k] = (float)(twd[k] - (double)twf[k]);
+      const double w[2] = {std::cos(ang), std::sin(ang)};
+      for (int k = 0; k < 2; ++k) {
+        if (single) {
+          tf[2 * t + k] = (float)w[k];
+          tf[2 * (n + t) + k] = (float)(w[k] - (double)(float)w[k]);
+        } else {
+          td[2 * t + k] = w[k];
+        }
       }
-      e = cudaMemcpy(p->tw_dev[i], twf.data(), 2 * wb * n, cudaMemcpyHostToDevice);
-      p->ax[i].tw_lo = (const float2*)p->tw_dev[i] + n;
     }
-    if (e != cudaSuccess) {
-      mmx_plan_destroy(p);
-      return cuda_fail(e, "cudaMemcpy(twiddles)");
-    }
-    p->ax[i].tw = p->tw_dev[i];
-    p->kv_off[i] = kv_total;
-    kv_total += n;
   }
-  // the k tables in the plan's precision, and behind them (complex64) the same in FP64
-  const size_t kv_bytes = ((wb / 2) * (size_t)kv_total + 15) & ~(size_t)15;
-  const size_t kv_all = kv_bytes + (precision == MMX_C64 ? sizeof(double) * (size_t)kv_total : 0);
-  cudaError_t e = cudaMalloc(&p->kv_dev, kv_all);
-  if (e == cudaSuccess) e = cudaMemset(p->kv_dev, 0, kv_all);
-  if (e == cudaSuccess && precision == MMX_C64) p->kvd_dev = (double*)((unsigned char*)p->kv_dev + kv_bytes);
+  unsigned char* base = nullptr;
+  cudaError_t e = cudaMalloc(&p->small, off + sizeof(double) * (size_t)p->partials_len);
+  if (e == cudaSuccess) e = cudaMemcpy(p->small, image.data(), off, cudaMemcpyHostToDevice);
   if (e == cudaSuccess) e = cudaMalloc(&p->work, wb * (size_t)batch * ncomp * p->N);
   if (e != cudaSuccess) {
     mmx_plan_destroy(p);
     return cuda_fail(e, "cudaMalloc(plan buffers)");
   }
+  base = (unsigned char*)p->small;
+  for (int i = 0; i < ndim; ++i) {
+    p->ax[i].tw = base + tw_off[i];
+    if (single) p->ax[i].tw_lo = (const float2*)(base + tw_off[i]) + shape[i];
+  }
+  p->kv_dev = base + kv_off;
+  if (single) p->kvd_dev = (double*)(base + kvd_off);
+  p->done = (unsigned int*)(base + done_off);
+  p->loop_counter = p->done + batch;
+  p->partials = (double*)(base + off);
   {
     const char* fg = getenv("MMX_FORCE_GENERIC");
     p->force_generic = fg && fg[0] == '1';
@@ -1320,17 +1332,6 @@ int mmx_plan_create(int ndim, const int64_t* shape, int ncomp, int batch, int pr
   p->defect_passes = build_passes(p, true);
   p->plane_passes = build_plane_passes(p);
   p->epro_passes = build_epro_passes(p);
-  int64_t maxt = 2048;  // enough partial sums for any tile width (at most one tile per pencil)
-  for (int i = 0; i < ndim; ++i) maxt = std::max<int64_t>(maxt, p->N / shape[i]);
-  p->partials_len = (int64_t)batch * maxt * 2;
-  e = cudaMalloc(&p->partials, sizeof(double) * p->partials_len);
-  if (e == cudaSuccess) e = cudaMalloc(&p->done, sizeof(unsigned int) * (batch + 2));
-  if (e == cudaSuccess) e = cudaMemset(p->done, 0, sizeof(unsigned int) * (batch + 2));
-  p->loop_counter = p->done + batch;
-  if (e != cudaSuccess) {
-    mmx_plan_destroy(p);
-    return cuda_fail(e, "cudaMalloc(partials)");
-  }
   for (auto& pc : p->iter_passes) {
     if (pc.smem > kSmemCap || pc.threads > 512) {
       mmx_plan_destroy(p);
@@ -1344,12 +1345,8 @@ int mmx_plan_create(int ndim, const int64_t* shape, int ncomp, int batch, int pr
 int mmx_plan_destroy(mmx_plan* p) {
   if (!p) return MMX_OK;
   drop_graphs_of(p);
-  for (int i = 0; i < 3; ++i)
-    if (p->tw_dev[i]) cudaFree(p->tw_dev[i]);
-  if (p->kv_dev) cudaFree(p->kv_dev);
+  if (p->small) cudaFree(p->small);
   if (p->work) cudaFree(p->work);
-  if (p->partials) cudaFree(p->partials);
-  if (p->done) cudaFree(p->done);
   if (p->l2_persist) {  // hand the persisting set-aside back
     cudaCtxResetPersistingL2Cache();
     cudaDeviceSetLimit(cudaLimitPersistingL2CacheSize, p->l2_prev_limit);
