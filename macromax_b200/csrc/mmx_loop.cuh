@@ -260,7 +260,19 @@ __global__ void __launch_bounds__(kLoopThreads, sizeof(R) == 4 ? 2 : 1) k_loop(c
   __syncthreads();
   bool any = false;
   for (int b = 0; b < B; ++b) any |= S[b].active != 0;
-  if (!any) return;  // the same in every CTA
+  auto leave = [&] {  // the last CTA to leave resets the counters
+    if (tid == 0) {
+      __threadfence();
+      if (atomicAdd(a.counter + 1, 1u) == gridDim.x - 1) {
+        a.counter[0] = 0u;
+        a.counter[1] = 0u;
+      }
+    }
+  };
+  if (!any) {  // the same in every CTA (or another has given up)
+    leave();
+    return;
+  }
   for (int b = tid; b < B; b += kLoopThreads) coef[b] = loop_coef<R>(S + b, a.inv_total_d);
 
   const bool worker = tid < kLoopWorkers;
@@ -489,13 +501,7 @@ __global__ void __launch_bounds__(kLoopThreads, sizeof(R) == 4 ? 2 : 1) k_loop(c
       for (int w = tid; w < B * kWords; w += kLoopThreads)
         reinterpret_cast<int*>(out)[w] = reinterpret_cast<const int*>(S + cur * B)[w];
   }
-  if (tid == 0) {  // the last CTA to leave resets the counters
-    __threadfence();
-    if (atomicAdd(a.counter + 1, 1u) == gridDim.x - 1) {
-      a.counter[0] = 0u;
-      a.counter[1] = 0u;
-    }
-  }
+  leave();
 }
 
 // ---------------------------------------------------------------------------------------------------------------

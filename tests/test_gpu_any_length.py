@@ -176,3 +176,35 @@ def test_projections_match_tensor_expressions(shape, dtype):
     assert np.linalg.norm(be.longitudinal_projection_ft(F).cpu().numpy()[:, 0] - ref) <= tol * np.linalg.norm(f)
     assert np.linalg.norm(be.transversal_projection_ft(F).cpu().numpy()[:, 0] - (f - ref)) <= tol * np.linalg.norm(f)
     assert np.linalg.norm(be.transversal_projection_ft(conj).cpu().numpy()[:, 0] - np.conj(f - ref)) <= tol * np.linalg.norm(f)
+
+
+def test_chunks_in_one_launch_on_two_streams():
+    """Two solves whose chunks are one launch each, queued on two streams without waiting: the fields of the solves alone."""
+    import torch
+    from macromax_b200 import Bound, Grid, _native as nat
+    from macromax_b200.batch import BatchSolution
+
+    def make(shape, dtype):
+        wl = _problem(shape, 1, 'scalar')
+        grid = Grid(shape=shape, step=wl['step'])
+        return BatchSolution(grid, wl['source'][None], wl['epsilon'], bound=Bound(grid, thickness=wl['bound_thickness']),
+                             vacuum_wavelength=wl['wavelength'], dtype=dtype)
+
+    cases = [((300, 420), np.complex64), ((256, 256), np.complex128)]
+    alone = [make(*c) for c in cases]
+    both = [make(*c) for c in cases]
+    for s in alone:
+        assert nat.load().mmx_plan_chunk_ends(s.engine.plan.handle, s.engine.chi_kind) == 1
+        for _ in range(4):
+            s.engine.iterate(30)
+            torch.cuda.synchronize()
+    streams = [torch.cuda.Stream() for _ in both]
+    torch.cuda.synchronize()
+    for _ in range(4):
+        for s, stream in zip(both, streams):
+            s.engine.iterate(30, stream=stream)
+    torch.cuda.synchronize()
+    for s, ref in zip(both, alone):
+        nat.check_stalled(s.state)
+        assert np.array_equal(s.iterations, ref.iterations)
+        assert np.array_equal(s.E, ref.E)
