@@ -387,8 +387,17 @@ def bench_ours(args, wl, rank, world, local, pg):
         print(json.dumps(line), flush=True)
 
 
+def passes_of(wl, variant=0) -> int:
+    """The variant flags whose passes a plan runs: the default (0, or with tensor-staged passes) is the fused epilogue (16)
+    for vector fields on 3D grids."""
+    variant = int(variant or 0)
+    vector = np.asarray(wl['source']).shape[-1 - len(wl['shape'])] == 3
+    return variant | 16 if variant in (0, 32) and vector and len(wl['shape']) == 3 else variant
+
+
 def traffic_per_iteration(wl, variant=0):
     """DRAM bytes of one iteration of this workload and kernel variant from the committed ncu capture (or None)."""
+    variant = passes_of(wl, variant)
     path = os.path.join(ROOT, 'profiles', 'traffic.json')
     try:
         with open(path) as f:
@@ -746,6 +755,7 @@ def len_passes(wl, variant=0) -> int:
 def fused_epilogue(wl, variant=0) -> bool:
     """Whether the plan runs the fused epilogue: isotropic chi, or a 3x3 chi on 192-sample rows of a vector field."""
     d = len(wl['shape'])
+    variant = passes_of(wl, variant)
     if d < 2 or not (variant or 0) & 16 or (variant or 0) & 8:
         return False
     iso = np.asarray(wl['epsilon']).ndim == d
