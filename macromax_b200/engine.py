@@ -25,16 +25,6 @@ def _complex_dtype(dtype):
     raise TypeError(f'unsupported dtype {dtype}: use complex64 or complex128')
 
 
-def _stream_ptr(stream=None):
-    s = stream if stream is not None else torch.cuda.current_stream()
-    return ctypes_void(s.cuda_stream)
-
-
-def ctypes_void(v):
-    import ctypes
-    return ctypes.c_void_p(int(v)) if v else None
-
-
 def _ptr(t: torch.Tensor):
     return nat.device_ptr(t)
 
