@@ -124,7 +124,8 @@ int mmx_iterate(mmx_plan* plan, void* E0, void* E1, const void* chi, int chi_kin
 /*
  * mmx_iterate for `niter` iterations as one CUDA graph launch: the pass kernels are captured once per (plan,
  * buffers, niter) and replayed, which removes the per-kernel launch gaps that dominate small grids.  Same
- * semantics as mmx_iterate.  The captured graph is released with the plan.
+ * semantics as mmx_iterate.  The captured graph is released with the plan.  Where a chunk runs in one launch
+ * (mmx_plan_chunk_ends) there is no graph, and the launch is cooperative: its blocks wait for one another.
  */
 int mmx_iterate_graph(mmx_plan* plan, void* E0, void* E1, const void* chi, int chi_kind, const void* src,
                       mmx_rhs_state* state, int niter, void* stream);
