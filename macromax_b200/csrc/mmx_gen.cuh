@@ -14,6 +14,8 @@
 // Strided tiles: P = 2^lP consecutive pencils, shared memory [component][sample][pencil]; a warp's accesses are whole
 // rows.  Contiguous tiles: P rows of every component, shared memory [row][sample] with a skew of one word per 128 bytes.
 #pragma once
+#include <cfloat>
+#include <math_constants.h>
 #include <type_traits>
 
 #include "mmx_dft.cuh"
@@ -132,9 +134,15 @@ __device__ __forceinline__ void gen_butterfly(int i, const GenAxis& g, int s, co
 
 // -i alpha_i / (|k|^2 - alpha) / N (solver.py:566-568, with the 1/N of the inverse transform), in FP64 and rounded once
 // (the field converges to the fixed point of the rounded g): complex64 starts the reciprocal in float and takes one
-// Newton step, about ten FP64 operations per sample.
+// Newton step, about ten FP64 operations per sample.  An alpha whose alpha_i^2 is beyond the range of R (an alpha that the
+// divergence guard has raised a hundred times) gives NaN, as the quotient in R does: every update is then rejected and the
+// residue stays infinite.  (A g of 0 would give an update of 0, which counts as converged.)
 template <class R> struct GenGreen {
   double ar, ai, ai2, s;
+  __device__ __forceinline__ GenGreen(double re, double im, double inv_total) : ar(re), ai(im), ai2(im * im), s(inv_total) {
+    // 1 / inf = 0 makes the Newton step 0 inf
+    if (sizeof(R) == 4 && ai2 > (double)FLT_MAX) ai2 = CUDART_INF;
+  }
   __device__ __forceinline__ cpx<R> operator()(double k2) const {
     const double dr = k2 - ar;
     const double den = fma(dr, dr, ai2);
@@ -270,7 +278,7 @@ __device__ __forceinline__ void green_tile(const GenAxis& g, int lP, int ndim, u
   const bool valid = p < inner;  // axis 0 has outer == 1: a pencil is its inner index
   cpx<R>* gp = T0 + p;
   const double kt2 = k1 * k1 + k2 * k2;
-  const GenGreen<R> green{ar, ai, ai * ai, inv_total};
+  const GenGreen<R> green(ar, ai, inv_total);
   auto component = [&](int& i, int T) {  // i in [0, C T) -> component, i mod T
     int c = 0;
     if constexpr (C == 3) {

@@ -134,7 +134,7 @@ __global__ void __launch_bounds__(LenGreen<R, C, N>::THREADS, (LenGreen<R, C, N>
   if (!st->active) return;
   cpx<R>* gp = a.T + (int64_t)blockIdx.y * C * a.N + p;
   const double kt2 = k1 * k1 + k2 * k2, ar = st->alpha_re, ai = st->alpha_im;
-  const GenGreen<R> green{ar, ai, ai * ai, a.inv_total_d};
+  const GenGreen<R> green(ar, ai, a.inv_total_d);
 #pragma unroll 1
   for (int e = slot; e < C * L::T0; e += SLOTS) {
     const int c = e / L::T0, i = e - c * L::T0;

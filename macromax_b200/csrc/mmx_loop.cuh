@@ -593,7 +593,7 @@ __global__ void __launch_bounds__(kLineThreads, 1) k_line(const __grid_constant_
     const ChiCoef<R> cc = chi_coef<R>(st);
     const double ar = st->alpha_re, ai = st->alpha_im, inv = a.inv_total_d;
     stages(std::integral_constant<int, -1>{});
-    const GenGreen<R> green{ar, ai, ai * ai, inv};
+    const GenGreen<R> green(ar, ai, inv);
     const cpx<R> h = C == 3 ? gen_longitudinal<R>(ar, ai, inv) : mkc<R>((R)0, (R)0);
     for (int j = tid; j < n; j += kLineThreads) {
       const double k0 = sk0[j];
