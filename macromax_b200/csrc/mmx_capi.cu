@@ -985,11 +985,16 @@ bool epro_runs(const mmx_plan* p, int chi_kind) {
 // complex64 300 x 420 14.3 / 30.0, 8 sources on 200 x 180 19.0 / 29.6, 48 x 42 x 44 18.5 / 30.6 (vector: 23.5 / 33.5);
 // specialised: 64^2 9.3 / 13.1, 256^2 11.9 / 18.0, 512^2 22.4 / 24.0, 64^3 20.0 / 18.8; complex128 64^2 8.7 / 20.8, 256^2
 // 11.7 / 32.9, 512^2 23.1 / 29.6, 64^3 27.0 / 34.8; 1000 samples in 1D 6.2 / 20.0 (complex128 6.6 / 24.2).
+// Vector fields on 1D grids keep the passes too: a field along the only axis has a local Green function, its solve is often at
+// rounding level after 15 to 35 iterations, and from there on rounding alone says which updates the guard rejects.  Each
+// rejection raises alpha for good, so the results of the next solve of the same object would be others.
+// MMX_VARIANT_LOOP takes the one launch.
 const LoopCfg* loop_runs(mmx_plan* p, int chi_kind) {
   if (p->force_generic || p->no_reg || p->pipe || p->plane || p->epro || p->tma || p->runtime_radix || p->passes_only ||
       p->compare_green || p->l2_persist)
     return nullptr;
   if (p->ncomp == 1 && chi_kind != MMX_CHI_SCALAR) return nullptr;
+  if (p->ndim == 1 && p->ncomp == 3 && !p->force_loop) return nullptr;
   if (p->ndim > 1 && !p->force_loop) {
     bool special = true;
     for (const PassCfg& pc : p->iter_passes) special &= pc.fast != 0;

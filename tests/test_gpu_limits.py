@@ -1,6 +1,6 @@
 """
-What the passes of the default variant do at the ends of their range, against the runtime-radix passes: an alpha that the
-divergence guard has raised beyond the range of the data type.
+What the default variant does at the ends of its range, against the runtime-radix passes: an alpha that the divergence
+guard has raised beyond the range of the data type, and solves from the alpha that an earlier solve left.
 """
 import numpy as np
 import pytest
@@ -34,3 +34,19 @@ def test_updates_are_rejected_when_alpha_is_out_of_range(shape, components, laun
         assert (s.iteration, s.rejections) == (5, 5)
         assert s._engine.read_state()['prev_norm'][0] == np.inf
         assert not np.any(s.E)
+
+
+@pytest.mark.parametrize('n', [200, 300, 420, 800])
+@pytest.mark.parametrize('dtype', [np.complex64, np.complex128])
+def test_repeated_solves_of_a_longitudinal_field(n, dtype):
+    """A 1D vector field along the axis converges to rounding level long before its 200 iterations end, and the rejections
+    that follow leave alpha raised: each of three solves in a row gives the field of the runtime-radix passes."""
+    from macromax_b200 import autotune
+    fast, gen = [_solution(_problem((n,), 3, 'scalar'), dtype) for _ in range(2)]
+    autotune.set_variant(gen._engine, _variants()['generic'])
+    for _ in range(3):
+        for s in (fast, gen):
+            s.E = 0.0
+            s.solve(None, rtol=0, maxiter=200)
+        assert (fast.iteration, fast.rejections, fast.alpha) == (gen.iteration, gen.rejections, gen.alpha)
+        assert np.array_equal(fast.E, gen.E)
