@@ -141,7 +141,8 @@ struct mmx_plan {
   double* partials = nullptr;
   int64_t partials_len = 0;
   unsigned int* done = nullptr;  // per-RHS tile counters of the epilogue pass (zero between iterations)
-  unsigned int* loop_counter = nullptr;  // the grid barrier of k_loop (two words, zero between launches)
+  unsigned int* loop_counter = nullptr;  // the grid barrier of k_loop (LEAVE_WORDS words, zero between launches)
+  unsigned loop_polls = kLoopPolls;      // of its waits (MMX_LOOP_POLL_LIMIT: fewer; tests)
   LoopCfg loop[3];             // chunks in one launch, per kind of chi (MMX_CHI_SCALAR, MMX_CHI_MAT3, MMX_CHI_SYM6)
   bool loop_known[3] = {false, false, false};
   bool passes_only = false;    // MMX_VARIANT_PASSES: no chunks in one launch
@@ -1020,7 +1021,7 @@ int run_loop(mmx_plan* p, const LoopCfg& cfg, void* E0, void* E1, const void* ch
   a.chi = (const cpx<R>*)chi;
   a.src = (const cpx<R>*)src;
   a.st = st;
-  MMX_CUDA(loop_launch<R>(cfg, a, p->ax, p->ncomp, chi_kind, p->batch, niter, p->loop_counter, s));
+  MMX_CUDA(loop_launch<R>(cfg, a, p->ax, p->ncomp, chi_kind, p->batch, niter, p->loop_polls, p->loop_counter, s));
   return MMX_OK;
 }
 
@@ -1264,7 +1265,7 @@ int mmx_plan_create(int ndim, const int64_t* shape, int ncomp, int batch, int pr
   const size_t kvd_off = off;
   if (single) off = up(off + sizeof(double) * (size_t)kv_total);
   const size_t done_off = off;
-  off = up(off + sizeof(unsigned int) * ((size_t)batch + 2));
+  off = up(off + sizeof(unsigned int) * ((size_t)batch + LEAVE_WORDS));
   int64_t maxt = 2048;  // enough partial sums for any tile width (at most one tile per pencil)
   for (int i = 0; i < ndim; ++i) maxt = std::max<int64_t>(maxt, p->N / shape[i]);
   p->partials_len = (int64_t)batch * maxt * 2;
@@ -1316,6 +1317,8 @@ int mmx_plan_create(int ndim, const int64_t* shape, int ncomp, int batch, int pr
     p->compare_green = wg && wg[0];
     const char* pl = getenv("MMX_PIPE_POLL_LIMIT");
     if (pl && pl[0]) p->poll_limit = std::max(0, std::min(1 << 20, atoi(pl)));
+    const char* ll = getenv("MMX_LOOP_POLL_LIMIT");
+    if (ll && ll[0]) p->loop_polls = (unsigned)std::max(0, std::min((int)kLoopPolls, atoi(ll)));
     const char* lp = getenv("MMX_L2_PERSIST");
     if (lp && lp[0] == '1' && precision == MMX_C64) {
       int maxp = 0, maxw = 0;

@@ -128,7 +128,7 @@ template <class R> LoopCfg loop_config(int ndim, const int64_t* shape, int C, in
 
 template <class R>
 cudaError_t loop_launch(const LoopCfg& cfg, const IterArgs<R>& base, const FFTAxis* tab, int C, int chi_kind, int B,
-                        int niter, unsigned* counter, cudaStream_t s) {
+                        int niter, unsigned polls, unsigned* counter, cudaStream_t s) {
   cudaLaunchConfig_t lc = {};
   lc.gridDim = dim3((unsigned)cfg.grid);
   lc.dynamicSmemBytes = cfg.smem;
@@ -160,6 +160,7 @@ cudaError_t loop_launch(const LoopCfg& cfg, const IterArgs<R>& base, const FFTAx
   a.PR = cfg.PR;
   a.kept = cfg.kept;
   a.niter = niter;
+  a.polls = polls;
   a.counter = counter;
   lc.blockDim = dim3(kLoopThreads);
   cudaLaunchAttribute attr[1];
@@ -175,9 +176,9 @@ cudaError_t loop_launch(const LoopCfg& cfg, const IterArgs<R>& base, const FFTAx
 #ifdef MMX_GEN_DOUBLE
 template LoopCfg loop_config<double>(int, const int64_t*, int, int, int, int);
 template cudaError_t loop_launch<double>(const LoopCfg&, const IterArgs<double>&, const FFTAxis*, int, int, int, int,
-                                         unsigned*, cudaStream_t);
+                                         unsigned, unsigned*, cudaStream_t);
 #else
 template LoopCfg loop_config<float>(int, const int64_t*, int, int, int, int);
-template cudaError_t loop_launch<float>(const LoopCfg&, const IterArgs<float>&, const FFTAxis*, int, int, int, int, unsigned*,
-                                        cudaStream_t);
+template cudaError_t loop_launch<float>(const LoopCfg&, const IterArgs<float>&, const FFTAxis*, int, int, int, int, unsigned,
+                                        unsigned*, cudaStream_t);
 #endif

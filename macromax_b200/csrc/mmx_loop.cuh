@@ -19,15 +19,16 @@
 // right-hand sides' prologue and first pass are done again from the old field.  When no right-hand side is active any
 // more the launch ends, so a chunk longer than the solve costs nothing.
 //
-// Waits: the grid barrier polls a counter at most kLoopPolls times, then marks every state MMX_STATUS_STALLED and
-// inactive and leaves.
+// Waits: a CTA polls the grid barrier's counter at most `polls` times (kLoopPolls; several seconds), then gives up and
+// leaves, and the others after it.  The last CTA to leave writes the states: those of the chunk's end, or, when any CTA gave
+// up, the old ones as MMX_STATUS_STALLED and inactive (mmx_leave.h).
 #pragma once
 #include "mmx_gen.cuh"
+#include "mmx_leave.h"
 
 constexpr int kLoopWorkers = 256;                // threads of a CTA that run the tiles
 constexpr int kLoopThreads = kLoopWorkers + 32;  // and the warp that takes the decisions
 constexpr int kLoopMaxRhs = 64;
-constexpr unsigned kLoopPolls = 1u << 24;
 
 template <class R> struct LoopArgs : IterArgs<R> {
   GenAxis g[3];     // axis 0, the middle axis of a 3D grid, the contiguous axis
@@ -36,7 +37,8 @@ template <class R> struct LoopArgs : IterArgs<R> {
   int tiles[3];     // per right-hand side (middle axis: per component)
   int kept;         // row tiles per CTA, at most
   int niter;
-  unsigned* counter;  // [0]: arrivals at the barrier, [1]: CTAs that have left (both 0 between launches)
+  unsigned polls;     // of a wait
+  unsigned* counter;  // LEAVE_WORDS words
 };
 
 enum : int { LOOP_EPI = 1, LOOP_PRO = 2 };
@@ -254,23 +256,31 @@ __global__ void __launch_bounds__(kLoopThreads, sizeof(R) == 4 ? 2 : 1) k_loop(c
   for (int w = tid; w < B * kWords; w += kLoopThreads)
     reinterpret_cast<int*>(S)[w] = reinterpret_cast<const int*>(a.st)[w];
   double* red = reinterpret_cast<double*>(mmx_smem_raw + lay.red);
-  volatile int* flags = reinterpret_cast<int*>(mmx_smem_raw + lay.flags);  // any active, any rejected, stalled
+  volatile int* flags = reinterpret_cast<int*>(mmx_smem_raw + lay.flags);  // any active, any rejected, stalled or last, -
   cpx<R>* kept = reinterpret_cast<cpx<R>*>(mmx_smem_raw + lay.kept);
   cpx<R>* sm = reinterpret_cast<cpx<R>*>(mmx_smem_raw + lay.work);
   __syncthreads();
   bool any = false;
   for (int b = 0; b < B; ++b) any |= S[b].active != 0;
-  auto leave = [&] {  // the last CTA to leave resets the counters
+  auto leave = [&](bool gave_up) {  // by the whole CTA; the last one clears the counters
+    __syncthreads();
     if (tid == 0) {
-      __threadfence();
-      if (atomicAdd(a.counter + 1, 1u) == gridDim.x - 1) {
-        a.counter[0] = 0u;
-        a.counter[1] = 0u;
-      }
+      const LeaveResult r = leave_launch(gridDim.x, gave_up, [&](int word, unsigned v) {
+        __threadfence();
+        const unsigned was = atomicAdd(a.counter + word, v);
+        __threadfence();
+        return was;
+      });
+      if (r.last)
+        for (int w = 0; w < LEAVE_WORDS; ++w) a.counter[w] = 0u;
+      flags[2] = r.last;
+      flags[3] = r.stalled;
     }
+    __syncthreads();
+    return LeaveResult{flags[2] != 0, flags[3] != 0};
   };
-  if (!any) {  // the same in every CTA (or another has given up)
-    leave();
+  if (!any) {  // the same in every CTA: nobody writes the states before all have left
+    leave(false);
     return;
   }
   for (int b = tid; b < B; b += kLoopThreads) coef[b] = loop_coef<R>(S + b, a.inv_total_d);
@@ -319,7 +329,7 @@ __global__ void __launch_bounds__(kLoopThreads, sizeof(R) == 4 ? 2 : 1) k_loop(c
         unsigned seen;
         asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(seen) : "l"(a.counter) : "memory");
         if ((int)(seen - want) >= 0) break;
-        if (polls == kLoopPolls) {
+        if (polls >= a.polls) {
           stalled = 1;
           break;
         }
@@ -481,13 +491,7 @@ __global__ void __launch_bounds__(kLoopThreads, sizeof(R) == 4 ? 2 : 1) k_loop(c
       ++pass;
     }
   }
-  mmx_rhs_state* out = const_cast<mmx_rhs_state*>(a.st);
-  if (!ok) {
-    for (int b = tid; b < B; b += kLoopThreads) {
-      atomicOr(&out[b].status, MMX_STATUS_STALLED);
-      out[b].active = 0;
-    }
-  } else {
+  if (ok) {
     each_row_tile([&](int k, int b, int tile) {
       const int64_t row0 = (int64_t)tile * a.PR, v0 = row0 * a.g[2].n;
       const int count = (int)(rows - row0 < a.PR ? rows - row0 : a.PR) * a.g[2].n;
@@ -497,11 +501,19 @@ __global__ void __launch_bounds__(kLoopThreads, sizeof(R) == 4 ? 2 : 1) k_loop(c
       for (int c = 0; c < C; ++c)
         for (int e = tid; e < count; e += kLoopThreads) E[c * N + e] = from[c * words + e];
     });
-    if (blockIdx.x == 0)
-      for (int w = tid; w < B * kWords; w += kLoopThreads)
-        reinterpret_cast<int*>(out)[w] = reinterpret_cast<const int*>(S + cur * B)[w];
   }
-  leave();
+  const LeaveResult r = leave(!ok);
+  if (!r.last) return;
+  mmx_rhs_state* out = const_cast<mmx_rhs_state*>(a.st);
+  if (r.stalled) {
+    for (int b = tid; b < B; b += kLoopThreads) {
+      out[b].status |= MMX_STATUS_STALLED;
+      out[b].active = 0;
+    }
+  } else {
+    for (int w = tid; w < B * kWords; w += kLoopThreads)
+      reinterpret_cast<int*>(out)[w] = reinterpret_cast<const int*>(S + cur * B)[w];
+  }
 }
 
 // ---------------------------------------------------------------------------------------------------------------

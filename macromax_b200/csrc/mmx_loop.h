@@ -1,6 +1,9 @@
 // Chunks of iterations in one launch (kernels: mmx_loop.cuh, launchers: mmx_loop.cu).
 #pragma once
 #include "mmx_gen.h"
+#include "mmx_leave.h"
+
+constexpr unsigned kLoopPolls = 1u << 24;  // of a wait between CTAs, unless the plan says otherwise
 
 struct LoopCfg {
   bool ok = false;
@@ -13,7 +16,7 @@ struct LoopCfg {
 // How a chunk of this plan's iterations runs in one launch; ok == false: it cannot.
 template <class R> LoopCfg loop_config(int ndim, const int64_t* shape, int C, int chi_kind, int B, int sms);
 
-// tab: the twiddle tables per grid axis; counter: two words, 0 between launches.
+// tab: the twiddle tables per grid axis; polls: of a wait between CTAs, at most; counter: LEAVE_WORDS words (mmx_leave.h).
 template <class R>
 cudaError_t loop_launch(const LoopCfg& cfg, const IterArgs<R>& a, const FFTAxis* tab, int C, int chi_kind, int B, int niter,
-                        unsigned* counter, cudaStream_t s);
+                        unsigned polls, unsigned* counter, cudaStream_t s);

@@ -1,12 +1,15 @@
 """
 What the default variant does at the ends of its range, against the runtime-radix passes: an alpha that the divergence
-guard has raised beyond the range of the data type, and solves from the alpha that an earlier solve left.
+guard has raised beyond the range of the data type, solves from the alpha that an earlier solve left, and waits between
+the blocks of a launch that run out.
 """
+import os
+
 import numpy as np
 import pytest
 
 from test_gpu_any_length import _problem
-from test_gpu_fast import _solution
+from test_gpu_fast import _solution, rel
 
 pytestmark = pytest.mark.gpu
 
@@ -50,3 +53,35 @@ def test_repeated_solves_of_a_longitudinal_field(n, dtype):
             s.solve(None, rtol=0, maxiter=200)
         assert (fast.iteration, fast.rejections, fast.alpha) == (gen.iteration, gen.rejections, gen.alpha)
         assert np.array_equal(fast.E, gen.E)
+
+
+@pytest.mark.parametrize('shape,components', [((300, 420), 1), ((36, 44, 39), 3)])
+@pytest.mark.parametrize('dtype', [np.complex64, np.complex128])
+def test_waits_that_run_out_are_reported(shape, components, dtype):
+    """The CTAs of a chunk in one launch look at the grid barrier once and give up: every state is marked, the host raises,
+    and the next launch of the plan starts from cleared counters."""
+    from macromax_b200 import _native as nat, autotune
+    wl = _problem(shape, components, 'scalar')
+    os.environ['MMX_LOOP_POLL_LIMIT'] = '0'
+    try:
+        sol = _solution(wl, dtype)
+    finally:
+        del os.environ['MMX_LOOP_POLL_LIMIT']
+    eng = sol._engine
+    autotune.set_variant(eng, nat.MMX_VARIANT_LOOP)
+    assert nat.load().mmx_plan_chunk_ends(eng.plan.handle, eng.chi_kind) == 1
+    for _ in range(2):
+        with pytest.raises(nat.NativeError):
+            sol.solve(None, rtol=0, maxiter=10)
+        st = eng.read_state()[0]
+        assert int(st['status']) == nat.MMX_STATUS_STALLED
+        assert (int(st['active']), int(st['iteration'])) == (0, 0)
+    # the same plan in passes, and another one whose waits may take their time
+    other = _solution(wl, dtype)
+    autotune.set_variant(other._engine, nat.MMX_VARIANT_LOOP)
+    autotune.set_variant(eng, nat.MMX_VARIANT_PASSES)
+    for s in (sol, other):
+        s.E = 0.0
+        s.solve(None, rtol=0, maxiter=10)
+        assert s.iteration == 10
+    assert rel(sol.E, other.E) < (1e-5 if dtype == np.complex64 else 1e-12)
