@@ -112,7 +112,6 @@ class BatchSolution:
         st = self.engine.run(float(rtol), float(maxiter))
         if np.any(st['status'] == nat.MMX_STATUS_ZERODIV):
             raise ZeroDivisionError('float division by zero (update norm after a zero update norm)')
-        nat.check_stalled(st)
         self._state = st
         return self
 
@@ -230,7 +229,10 @@ class UnevenBatch:
             m.engine.write_state(st)
         while True:
             self.iterate(chunk)
-            if not any(np.any(m.engine.read_state()['active']) for m in self.members):
+            states = [m.engine.read_state() for m in self.members]
+            for st in states:
+                nat.check_stalled(st)
+            if not any(np.any(st['active']) for st in states):
                 break
             chunk = min(2 * chunk, max_chunk)
         return self

@@ -264,6 +264,7 @@ class IterationEngine:
                 cont = True
                 todo -= n
             st = self.read_state()
+            nat.check_stalled(st)
             if not np.any(st['active']):
                 break
             look = look if whole else min(look * 2, max_chunk)

@@ -228,7 +228,10 @@ class MixedUnevenSolution:
             chunk = 8
             while True:
                 self._uneven.iterate(chunk)
-                if not any(np.any(m.inner.engine.read_state()['active']) for m in self.members):
+                states = [m.inner.engine.read_state() for m in self.members]
+                for st in states:
+                    nat.check_stalled(st)
+                if not any(np.any(st['active']) for st in states):
                     break
                 chunk = min(2 * chunk, 64)
             for m, f in zip(self.members, finished):

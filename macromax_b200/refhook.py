@@ -226,6 +226,7 @@ class _FusedRunner:
 
     def sync_out(self, sol, st):
         """Point the solution at the engine's current field and copy back the update norm, residue and alpha."""
+        nat.check_stalled(st)
         cur = int(st['cur'][0])
         view = self.engine.fields[cur, 0].view(self.ncomp, 1, *self.shape)
         sol._Solution__field_array = view
