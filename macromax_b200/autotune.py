@@ -107,11 +107,13 @@ def tune(engine, iters: int = 20, use_cache: bool = True, candidates=CANDIDATES)
     if not trials:
         engine.fields.copy_(fields)
         engine.state.copy_(state)
+        engine.state_written()
         raise RuntimeError('autotune: no variant ran its iterations on every right-hand side '
                            '(zero sources, or a diverging state?)')
     best = min(trials, key=trials.get)
     engine.fields.copy_(fields)
     engine.state.copy_(state)
+    engine.state_written()
     set_variant(engine, int(best))
     result = {'variant': int(best), 'us_per_iteration': trials[best], 'trials': trials}
     if use_cache:

@@ -216,6 +216,8 @@ class UnevenBatch:
     def iterate(self, niter: int):
         import ctypes
         s = torch.cuda.current_stream().cuda_stream
+        for m in self.members:
+            m.engine.state_written()
         nat.call('mmx_iterate_multi', *self._args, int(niter), ctypes.c_void_p(s) if s else None)
 
     def solve(self, rtol: float = 1e-6, maxiter=1e4, chunk: int = 8, max_chunk: int = 64) -> 'UnevenBatch':

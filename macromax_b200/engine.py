@@ -80,7 +80,7 @@ class IterationEngine:
             self.fields = torch.zeros((2, self.batch, self.ncomp, self.N), dtype=self.torch_dtype, device=self.device)
             self.sources = torch.zeros((self.batch, self.ncomp, self.N), dtype=self.torch_dtype, device=self.device)
             self.state = torch.zeros((self.batch, nat.STATE_DTYPE.itemsize), dtype=torch.uint8, device=self.device)
-        self._launches = 0  # iteration calls so far: with the state tensor's version, what a copy of the state is of
+        self._writes = 0  # of the states, by iteration calls and by the host (state_key)
         self.set_chi(chi0, alpha0)
         st = np.zeros(self.batch, dtype=nat.STATE_DTYPE)
         st['alpha_re'] = st['alpha0_re'] = alpha0.real
@@ -164,12 +164,18 @@ class IterationEngine:
         return host.view(nat.STATE_DTYPE).copy()
 
     def state_key(self):
-        """Changes with every iteration call and with every write to the state tensor."""
-        return self._launches, self.state._version
+        """Changes with every iteration call and with every write to the state tensor (one made under inference mode has
+        no version: who writes it other than by ``write_state`` calls ``state_written``)."""
+        return self._writes, None if self.state.is_inference() else self.state._version
+
+    def state_written(self):
+        """The states have been written other than by ``iterate`` and ``write_state``."""
+        self._writes += 1
 
     def write_state(self, st: np.ndarray):
         raw = np.ascontiguousarray(st, dtype=nat.STATE_DTYPE).view(np.uint8).reshape(self.batch, -1)
         self.state.copy_(torch.from_numpy(raw.copy()))
+        self._writes += 1
 
     def reset_alpha(self, index=None):
         """Return alpha to alpha0 (the stored chi and sources), e.g. before solving a new, unrelated problem."""
@@ -216,7 +222,7 @@ class IterationEngine:
         graph of ``niter`` iterations (a length that comes again)."""
         if niter <= 0:
             return
-        self._launches += 1
+        self._writes += 1
         if self.use_graphs and niter > 1 and graph:
             fn = 'mmx_iterate_graph_continue' if cont else 'mmx_iterate_graph'
         else:

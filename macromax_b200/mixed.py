@@ -102,6 +102,7 @@ class MixedSolution:
         finally:
             eng.sources.copy_(saved_src)
             eng.state.copy_(saved_state)
+            eng.state_written()
 
     def _xnorms(self) -> np.ndarray:
         """FP64 norms of every right-hand side's x, read back once (the launches queue on one stream and share the
