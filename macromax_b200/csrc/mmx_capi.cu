@@ -966,17 +966,18 @@ template <class R> IterArgs<R> base_args(mmx_plan* p) {
 // (us per iteration, plain and fused: 64^3 28.7 / 26.5, four sources 66.7 / 63.5; 128^3 119.7 / 109.5, four sources 482 /
 // 462; 192^3 with a 3x3 chi 555 / 490).  On 2D grids and for scalar fields it is not faster (128^3 scalar 47.1 / 50.5, 64
 // sources on 512^2 264 / 297): their passes hold less work per sample to hide its longer dependent chain behind.
-bool epro_chosen(const mmx_plan* p) {
+// A call of one iteration (a callback after each) has no next one to prepare for: plain passes there too.
+bool epro_chosen(const mmx_plan* p, int niter) {
   if (p->epro) return true;
-  return p->ncomp == 3 && p->ndim == 3 && !p->force_generic && !p->no_reg && !p->pipe && !p->plane &&
+  return niter > 1 && p->ncomp == 3 && p->ndim == 3 && !p->force_generic && !p->no_reg && !p->pipe && !p->plane &&
          !p->runtime_radix && !p->passes_only && !p->compare_green && !p->l2_persist;
 }
 
-// whether run_iterations takes the fused-epilogue schedule for this plan and chi
-bool epro_runs(const mmx_plan* p, int chi_kind) {
+// whether run_iterations takes the fused-epilogue schedule for this plan, chi and number of iterations
+bool epro_runs(const mmx_plan* p, int chi_kind, int niter) {
   if (p->prec != MMX_C64) return false;
   const bool plane = p->plane && chi_kind == MMX_CHI_SCALAR && !p->plane_passes.empty();
-  return !plane && epro_chosen(p) && epro_serves(p, chi_kind);
+  return !plane && epro_chosen(p, niter) && epro_serves(p, chi_kind);
 }
 
 // The configuration under which a chunk of iterations runs in one launch, or null.  It does in the default variant where
@@ -1028,17 +1029,17 @@ int run_loop(mmx_plan* p, const LoopCfg& cfg, void* E0, void* E1, const void* ch
 // record the buffers of an iteration call just launched on the stream (the record is cleared unless the call ran
 // the fused-epilogue schedule; later calls on the stream run after it)
 void note_iteration_call(mmx_plan* p, const void* E0, const void* E1, const void* chi, int chi_kind, const void* src,
-                         const void* st) {
-  p->cont_valid = epro_runs(p, chi_kind);
+                         const void* st, int niter) {
+  p->cont_valid = epro_runs(p, chi_kind, niter);
   const void* b[5] = {E0, E1, chi, src, st};
   for (int i = 0; i < 5; ++i) p->cont_buf[i] = b[i];
   p->cont_kind = chi_kind;
 }
 
 bool can_continue(const mmx_plan* p, const void* E0, const void* E1, const void* chi, int chi_kind, const void* src,
-                  const void* st) {
+                  const void* st, int niter) {
   const void* b[5] = {E0, E1, chi, src, st};
-  if (!p->cont_valid || p->cont_kind != chi_kind || !epro_runs(p, chi_kind)) return false;
+  if (!p->cont_valid || p->cont_kind != chi_kind || !epro_runs(p, chi_kind, niter)) return false;
   for (int i = 0; i < 5; ++i)
     if (p->cont_buf[i] != b[i]) return false;
   return true;
@@ -1058,7 +1059,7 @@ int run_iterations(mmx_plan* p, void* E0, void* E1, const void* chi, int chi_kin
   // the accept/reject decision is taken by the last tile of the epilogue pass (no separate launch)
   const bool plane = std::is_same<R, float>::value && p->plane && chi_kind == MMX_CHI_SCALAR &&
                      !p->plane_passes.empty();
-  const bool epro = std::is_same<R, float>::value && !plane && epro_chosen(p) && epro_serves(p, chi_kind);
+  const bool epro = std::is_same<R, float>::value && !plane && epro_chosen(p, niter) && epro_serves(p, chi_kind);
   if (epro) {
     // first prologue of the chunk, then per iteration the middle passes, the fused epilogue + next prologue and
     // the repair pass
@@ -1420,7 +1421,7 @@ int mmx_iterate(mmx_plan* p, void* E0, void* E1, const void* chi, int chi_kind, 
   }
   const int rc = p->prec == MMX_C128 ? run_iterations<double>(p, E0, E1, chi, chi_kind, src, state, niter, s)
                                      : run_iterations<float>(p, E0, E1, chi, chi_kind, src, state, niter, s);
-  if (rc == MMX_OK && niter > 0) note_iteration_call(p, E0, E1, chi, chi_kind, src, state);
+  if (rc == MMX_OK && niter > 0) note_iteration_call(p, E0, E1, chi, chi_kind, src, state, niter);
   return rc;
 }
 
@@ -1603,7 +1604,7 @@ int iterate_multi(int n, mmx_plan* const* plans, void* const* E0, void* const* E
     return MMX_OK;
   }
   key.ints.push_back(niter);
-  const bool skip = cont && n == 1 && can_continue(plans[0], E0[0], E1[0], chi[0], chi_kind[0], src[0], state[0]);
+  const bool skip = cont && n == 1 && can_continue(plans[0], E0[0], E1[0], chi[0], chi_kind[0], src[0], state[0], niter);
   // a prepared continuation also captures the self-contained graph; a launch takes the one that applies
   for (int variant = (!launch && skip) ? 0 : (skip ? 1 : 0); variant <= (skip ? 1 : 0); ++variant) {
     GraphKey k = key;
@@ -1630,7 +1631,8 @@ int iterate_multi(int n, mmx_plan* const* plans, void* const* E0, void* const* E
     if (launch) {
       for (int i = 0; i < n; ++i) plans[i]->cont_valid = false;
       MMX_CUDA(cudaGraphLaunch(exec, (cudaStream_t)stream));
-      for (int i = 0; i < n; ++i) note_iteration_call(plans[i], E0[i], E1[i], chi[i], chi_kind[i], src[i], state[i]);
+      for (int i = 0; i < n; ++i)
+        note_iteration_call(plans[i], E0[i], E1[i], chi[i], chi_kind[i], src[i], state[i], niter);
     }
   }
   return MMX_OK;
