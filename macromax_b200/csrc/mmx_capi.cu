@@ -966,10 +966,12 @@ template <class R> IterArgs<R> base_args(mmx_plan* p) {
 // (us per iteration, plain and fused: 64^3 28.7 / 26.5, four sources 66.7 / 63.5; 128^3 119.7 / 109.5, four sources 482 /
 // 462; 192^3 with a 3x3 chi 555 / 490).  On 2D grids and for scalar fields it is not faster (128^3 scalar 47.1 / 50.5, 64
 // sources on 512^2 264 / 297): their passes hold less work per sample to hide its longer dependent chain behind.
-// A call of one iteration (a callback after each) has no next one to prepare for: plain passes there too.
+// Calls of one or two iterations (a callback after each) keep the plain passes as well: the last fused epilogue of a call
+// prepares an iteration that starts with its own first pass (us per iteration in calls of 1, 2, 3 and 4, fused against plain:
+// 64^3 33.4, 30.5, 29.6, 29.0 / 30.2; 128^3 137.2, 124.1, 119.6, 117.3 / 121.2; 192^3 with a 3x3 chi 641, 565, 540, 527 / 553).
 bool epro_chosen(const mmx_plan* p, int niter) {
   if (p->epro) return true;
-  return niter > 1 && p->ncomp == 3 && p->ndim == 3 && !p->force_generic && !p->no_reg && !p->pipe && !p->plane &&
+  return niter > 2 && p->ncomp == 3 && p->ndim == 3 && !p->force_generic && !p->no_reg && !p->pipe && !p->plane &&
          !p->runtime_radix && !p->passes_only && !p->compare_green && !p->l2_persist;
 }
 

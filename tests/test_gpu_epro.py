@@ -206,23 +206,24 @@ def test_continued_chunks_with_rejections_follow_the_oracle():
 
 
 @pytest.mark.parametrize('matrix', [False, True])
-def test_single_iterations_take_the_plain_passes(matrix):
-    """One iteration at a time, as with a callback, has no next one to prepare for: the plain schedule in the default
-    variant; and a chunk that is said to go on from a single iteration starts with its own first pass."""
+@pytest.mark.parametrize('step', [1, 2])
+def test_single_iterations_take_the_plain_passes(matrix, step):
+    """One or two iterations at a time, as with a callback, are too few for the fused epilogue: the plain schedule in the
+    default variant; and a chunk that is said to go on from them starts with its own first pass."""
     from macromax_b200 import _native as nat, autotune, workloads as w
     from test_gpu_fast import _solution, _stacked_voronoi
     wl = _stacked_voronoi(2) if matrix else w.spheres_3d(n=64, nb_spheres=40)
     sols = [_solution(wl) for _ in range(2)]
     autotune.set_variant(sols[1]._engine, nat.MMX_VARIANT_PASSES)
     for s in sols:
-        for _ in range(6):
-            s._engine.iterate(1)
+        for _ in range(6 // step):
+            s._engine.iterate(step)
     assert sols[0].iteration == sols[1].iteration == 6
     assert np.array_equal(sols[0].E, sols[1].E)
     autotune.set_variant(sols[1]._engine, 0)
     for s, cont in zip(sols, (True, False)):
         s._engine.iterate(4)
-        s._engine.iterate(1, cont=cont)
+        s._engine.iterate(step, cont=cont)
         s._engine.iterate(4, cont=cont)
-    assert sols[0].iteration == sols[1].iteration == 15
+    assert sols[0].iteration == sols[1].iteration == 14 + step
     assert np.array_equal(sols[0].E, sols[1].E)
