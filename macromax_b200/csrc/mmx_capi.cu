@@ -147,6 +147,7 @@ struct mmx_plan {
   bool loop_known[3] = {false, false, false};
   bool passes_only = false;    // MMX_VARIANT_PASSES: no chunks in one launch
   bool force_loop = false;     // MMX_VARIANT_LOOP: chunks in one launch at any size that they take
+  int loop_sms = 0;            // MMX_LOOP_SMS: SMs that they count on (0: those of the device; tests)
   std::vector<PassCfg> iter_passes;
   std::vector<PassCfg> defect_passes;
   bool force_generic = false;  // MMX_FORCE_GENERIC=1: use only the runtime-length kernels (tests)
@@ -993,7 +994,7 @@ bool epro_runs(const mmx_plan* p, int chi_kind, int niter) {
 // rounding level after 15 to 35 iterations, and from there on rounding alone says which updates the guard rejects.  Each
 // rejection raises alpha for good, so the results of the next solve of the same object would be others.
 // MMX_VARIANT_LOOP takes the one launch.
-const LoopCfg* loop_runs(mmx_plan* p, int chi_kind) {
+LoopCfg* loop_runs(mmx_plan* p, int chi_kind) {
   if (p->force_generic || p->no_reg || p->pipe || p->plane || p->epro || p->tma || p->runtime_radix || p->passes_only ||
       p->compare_green || p->l2_persist)
     return nullptr;
@@ -1006,8 +1007,9 @@ const LoopCfg* loop_runs(mmx_plan* p, int chi_kind) {
   }
   const int k = chi_kind == MMX_CHI_SCALAR ? 0 : chi_kind == MMX_CHI_MAT3 ? 1 : 2;
   if (!p->loop_known[k]) {
-    p->loop[k] = p->prec == MMX_C128 ? loop_config<double>(p->ndim, p->shape, p->ncomp, chi_kind, p->batch, sm_count())
-                                     : loop_config<float>(p->ndim, p->shape, p->ncomp, chi_kind, p->batch, sm_count());
+    const int sms = p->loop_sms ? p->loop_sms : sm_count();
+    p->loop[k] = p->prec == MMX_C128 ? loop_config<double>(p->ndim, p->shape, p->ncomp, chi_kind, p->batch, sms)
+                                     : loop_config<float>(p->ndim, p->shape, p->ncomp, chi_kind, p->batch, sms);
     // the contiguous-axis tiles' partial sums
     if ((int64_t)p->batch * p->loop[k].tiles[2] * 2 > p->partials_len) p->loop[k].ok = false;
     p->loop_known[k] = true;
@@ -1015,8 +1017,11 @@ const LoopCfg* loop_runs(mmx_plan* p, int chi_kind) {
   return p->loop[k].ok ? &p->loop[k] : nullptr;
 }
 
+// A chunk in one launch.  A context that cannot hold all its CTAs at once (one with a part of the SMs) refuses the launch:
+// then this plan's chunks run in passes from now on, and the caller's is still to be run (kLoopRefused).
+constexpr int kLoopRefused = 1;
 template <class R>
-int run_loop(mmx_plan* p, const LoopCfg& cfg, void* E0, void* E1, const void* chi, int chi_kind, const void* src,
+int run_loop(mmx_plan* p, LoopCfg& cfg, void* E0, void* E1, const void* chi, int chi_kind, const void* src,
              mmx_rhs_state* st, int niter, cudaStream_t s) {
   IterArgs<R> a = base_args<R>(p);
   a.E0 = (cpx<R>*)E0;
@@ -1024,8 +1029,20 @@ int run_loop(mmx_plan* p, const LoopCfg& cfg, void* E0, void* E1, const void* ch
   a.chi = (const cpx<R>*)chi;
   a.src = (const cpx<R>*)src;
   a.st = st;
-  MMX_CUDA(loop_launch<R>(cfg, a, p->ax, p->ncomp, chi_kind, p->batch, niter, p->loop_polls, p->loop_counter, s));
+  const cudaError_t e = loop_launch<R>(cfg, a, p->ax, p->ncomp, chi_kind, p->batch, niter, p->loop_polls, p->loop_counter, s);
+  if (!cfg.line && (e == cudaErrorCooperativeLaunchTooLarge || e == cudaErrorNotSupported)) {
+    cudaGetLastError();
+    cfg.ok = false;
+    return kLoopRefused;
+  }
+  MMX_CUDA(e);
   return MMX_OK;
+}
+
+int run_loop(mmx_plan* p, LoopCfg& cfg, void* E0, void* E1, const void* chi, int chi_kind, const void* src,
+             mmx_rhs_state* st, int niter, cudaStream_t s) {
+  return p->prec == MMX_C128 ? run_loop<double>(p, cfg, E0, E1, chi, chi_kind, src, st, niter, s)
+                             : run_loop<float>(p, cfg, E0, E1, chi, chi_kind, src, st, niter, s);
 }
 
 // record the buffers of an iteration call just launched on the stream (the record is cleared unless the call ran
@@ -1322,6 +1339,8 @@ int mmx_plan_create(int ndim, const int64_t* shape, int ncomp, int batch, int pr
     if (pl && pl[0]) p->poll_limit = std::max(0, std::min(1 << 20, atoi(pl)));
     const char* ll = getenv("MMX_LOOP_POLL_LIMIT");
     if (ll && ll[0]) p->loop_polls = (unsigned)std::max(0, std::min((int)kLoopPolls, atoi(ll)));
+    const char* ls = getenv("MMX_LOOP_SMS");
+    if (ls && ls[0]) p->loop_sms = std::max(0, std::min(1 << 16, atoi(ls)));
     const char* lp = getenv("MMX_L2_PERSIST");
     if (lp && lp[0] == '1' && precision == MMX_C64) {
       int maxp = 0, maxw = 0;
@@ -1417,9 +1436,10 @@ int mmx_iterate(mmx_plan* p, void* E0, void* E1, const void* chi, int chi_kind, 
   cudaStream_t s = (cudaStream_t)stream;
   p->cont_valid = false;
   if (niter > 0) {
-    if (const LoopCfg* loop = loop_runs(p, chi_kind))
-      return p->prec == MMX_C128 ? run_loop<double>(p, *loop, E0, E1, chi, chi_kind, src, state, niter, s)
-                                 : run_loop<float>(p, *loop, E0, E1, chi, chi_kind, src, state, niter, s);
+    if (LoopCfg* loop = loop_runs(p, chi_kind)) {
+      const int rc = run_loop(p, *loop, E0, E1, chi, chi_kind, src, state, niter, s);
+      if (rc != kLoopRefused) return rc;
+    }
   }
   const int rc = p->prec == MMX_C128 ? run_iterations<double>(p, E0, E1, chi, chi_kind, src, state, niter, s)
                                      : run_iterations<float>(p, E0, E1, chi, chi_kind, src, state, niter, s);
@@ -1595,12 +1615,12 @@ int iterate_multi(int n, mmx_plan* const* plans, void* const* E0, void* const* E
     if (!launch) return MMX_OK;
     for (int i : loops) {
       mmx_plan* p = plans[i];
-      const LoopCfg& loop = *loop_runs(p, chi_kind[i]);
       p->cont_valid = false;
-      const cudaStream_t s = (cudaStream_t)stream;
-      const int code = p->prec == MMX_C128
-                           ? run_loop<double>(p, loop, E0[i], E1[i], chi[i], chi_kind[i], src[i], state[i], niter, s)
-                           : run_loop<float>(p, loop, E0[i], E1[i], chi[i], chi_kind[i], src[i], state[i], niter, s);
+      int code = kLoopRefused;
+      if (LoopCfg* loop = loop_runs(p, chi_kind[i]))  // (a plan given twice may have been refused)
+        code = run_loop(p, *loop, E0[i], E1[i], chi[i], chi_kind[i], src[i], state[i], niter, (cudaStream_t)stream);
+      if (code == kLoopRefused)
+        code = iterate_multi(1, plans + i, E0 + i, E1 + i, chi + i, chi_kind + i, src + i, state + i, niter, stream, true);
       if (code != MMX_OK) return code;
     }
     return MMX_OK;

@@ -1,7 +1,7 @@
 """
 What the default variant does at the ends of its range, against the runtime-radix passes: an alpha that the divergence
 guard has raised beyond the range of the data type, solves from the alpha that an earlier solve left, and waits between
-the blocks of a launch that run out.
+the blocks of a launch that run out or cannot be made.
 """
 import os
 
@@ -85,3 +85,39 @@ def test_waits_that_run_out_are_reported(shape, components, dtype):
         s.solve(None, rtol=0, maxiter=10)
         assert s.iteration == 10
     assert rel(sol.E, other.E) < (1e-5 if dtype == np.complex64 else 1e-12)
+
+
+@pytest.mark.parametrize('shape,components,batch', [((640, 600), 1, 1), ((80, 78, 77), 1, 1), ((300, 420), 1, 4)])
+def test_refused_launches_run_in_passes(shape, components, batch):
+    """Where the blocks of a chunk in one launch cannot all run at once the launch is refused: the chunk runs in passes
+    instead, also as a member of an uneven batch, and so do the plan's later ones."""
+    from macromax_b200 import Bound, Grid, _native as nat, autotune
+    from macromax_b200.batch import BatchSolution, UnevenBatch
+    wl = _problem(shape, components, 'scalar')
+    grid = Grid(shape=shape, step=wl['step'])
+
+    def make():
+        return BatchSolution(grid, np.stack([wl['source']] * batch), wl['epsilon'], vacuum_wavelength=wl['wavelength'],
+                             bound=Bound(grid, thickness=wl['bound_thickness']))
+
+    def one_launch(s):
+        return nat.load().mmx_plan_chunk_ends(s.engine.plan.handle, s.engine.chi_kind)
+
+    os.environ['MMX_LOOP_SMS'] = '4096'
+    try:
+        sols = [make() for _ in range(3)]
+    finally:
+        del os.environ['MMX_LOOP_SMS']
+    ref = make()
+    assert one_launch(ref) == 1
+    autotune.set_variant(ref.engine, nat.MMX_VARIANT_PASSES)
+    ref.solve(rtol=0, maxiter=10)
+    assert all(one_launch(s) == 1 for s in sols)
+    sols[0].solve(rtol=0, maxiter=10)
+    for _ in range(10):
+        sols[1].iterate(1)
+    UnevenBatch(sols[2:]).solve(rtol=0, maxiter=10)
+    for s in sols:
+        assert one_launch(s) == 0
+        assert np.all(s.iterations == 10) and np.all(s.state['status'] == 0)
+        assert np.array_equal(s.E, ref.E)
