@@ -161,7 +161,6 @@ struct mmx_plan {
   bool epro = false;           // fuse each epilogue with the next iteration's prologue
   bool tma = false;            // strided 128-sample passes staged by bulk tensor copies (k_tma_pass)
   bool runtime_radix = false;  // k_iter_pass instead of the any-length passes (MMX_VARIANT_RUNTIME_RADIX)
-  bool compare_green = false;  // MMX_WIDE_GREEN set, to 0 or 1: the axis-0 pass's tiles are compared, so it has to run
   bool wide_green = false;     // MMX_WIDE_GREEN=1: 16-pencil tiles for the vector axis-0 pass (tests)
   std::vector<PassCfg> epro_passes;   // [middle passes..., EPI+PRO, repair]; the first PRO runs once per call
   // The last iteration call on this plan whose fused epilogue left the next iteration's first pass (the prologue
@@ -973,7 +972,7 @@ template <class R> IterArgs<R> base_args(mmx_plan* p) {
 bool epro_chosen(const mmx_plan* p, int niter) {
   if (p->epro) return true;
   return niter > 2 && p->ncomp == 3 && p->ndim == 3 && !p->force_generic && !p->no_reg && !p->pipe && !p->plane &&
-         !p->runtime_radix && !p->passes_only && !p->compare_green && !p->l2_persist;
+         !p->runtime_radix && !p->passes_only && !p->l2_persist;
 }
 
 // whether run_iterations takes the fused-epilogue schedule for this plan, chi and number of iterations
@@ -996,7 +995,7 @@ bool epro_runs(const mmx_plan* p, int chi_kind, int niter) {
 // MMX_VARIANT_LOOP takes the one launch.
 LoopCfg* loop_runs(mmx_plan* p, int chi_kind) {
   if (p->force_generic || p->no_reg || p->pipe || p->plane || p->epro || p->tma || p->runtime_radix || p->passes_only ||
-      p->compare_green || p->l2_persist)
+      p->l2_persist)
     return nullptr;
   if (p->ncomp == 1 && chi_kind != MMX_CHI_SCALAR) return nullptr;
   if (p->ndim == 1 && p->ncomp == 3 && !p->force_loop) return nullptr;
@@ -1334,7 +1333,6 @@ int mmx_plan_create(int ndim, const int64_t* shape, int ncomp, int batch, int pr
     p->pipe = pp && pp[0] == '1';
     const char* wg = getenv("MMX_WIDE_GREEN");
     p->wide_green = wg && wg[0] == '1';
-    p->compare_green = wg && wg[0];
     const char* pl = getenv("MMX_PIPE_POLL_LIMIT");
     if (pl && pl[0]) p->poll_limit = std::max(0, std::min(1 << 20, atoi(pl)));
     const char* ll = getenv("MMX_LOOP_POLL_LIMIT");

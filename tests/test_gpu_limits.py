@@ -121,3 +121,31 @@ def test_refused_launches_run_in_passes(shape, components, batch):
         assert one_launch(s) == 0
         assert np.all(s.iterations == 10) and np.all(s.state['status'] == 0)
         assert np.array_equal(s.E, ref.E)
+
+
+@pytest.mark.parametrize('wide', ['0', '1'])
+def test_tile_width_leaves_the_schedule_alone(wide):
+    """MMX_WIDE_GREEN chooses the tiles of the vector axis-0 pass and nothing else: a grid whose chunks run in one launch
+    keeps them, a grid with the fused epilogue has its bits; and the pass itself, reached with MMX_VARIANT_PASSES, gives the
+    same bits with both tile widths."""
+    from macromax_b200 import _native as nat, autotune, workloads as w
+    ragged = _problem((128, 40, 45), 3, 'scalar')
+    box = w.spheres_3d(n=128, nb_spheres=20)
+    box = {**box, 'shape': (128, 64, 64), 'epsilon': box['epsilon'][:, :64, :64], 'source': box['source'][..., :64, :64]}
+    sols = {}
+    for name, env in (('set', wide), ('unset', None)):
+        if env is not None:
+            os.environ['MMX_WIDE_GREEN'] = env
+        try:
+            sols[name] = [_solution(x) for x in (ragged, box, box)]
+        finally:
+            os.environ.pop('MMX_WIDE_GREEN', None)
+        autotune.set_variant(sols[name][2]._engine, nat.MMX_VARIANT_PASSES)
+    for a, b in zip(sols['set'], sols['unset']):
+        ends = [nat.load().mmx_plan_chunk_ends(s._engine.plan.handle, s._engine.chi_kind) for s in (a, b)]
+        assert ends[0] == ends[1]
+        for s in (a, b):
+            s.solve(None, rtol=0, maxiter=12)
+        assert np.array_equal(a.E, b.E)
+    one = sols['unset'][0]._engine
+    assert nat.load().mmx_plan_chunk_ends(one.plan.handle, one.chi_kind) == 1
