@@ -601,6 +601,7 @@ __global__ void __launch_bounds__(kLineThreads, 1) k_line(const __grid_constant_
     __syncthreads();
   };
   input();
+  int side = st->cur;  // of E
   for (int it = 0; it < a.niter; ++it) {
     const ChiCoef<R> cc = chi_coef<R>(st);
     const double ar = st->alpha_re, ai = st->alpha_im, inv = a.inv_total_d;
@@ -643,12 +644,13 @@ __global__ void __launch_bounds__(kLineThreads, 1) k_line(const __grid_constant_
     worker_sums(dd2, en2, red, sums, BlockSync());
     if (tid == 0) apply_decision(st, sums[0], sums[1]);
     __syncthreads();
-    if (st->accepted) {
+    if (st->cur != side) {  // (a state that ends with a status keeps `accepted` and its field)
+      side ^= 1;
       cpx<R>* t = E;
       E = En;
       En = t;
     }
-    if (!st->active) break;  // (with a status, the previous field)
+    if (!st->active) break;
     if (!st->accepted) input();
   }
   cpx<R>* to = (st->cur ? a.E1 : a.E0) + f;

@@ -149,3 +149,26 @@ def test_tile_width_leaves_the_schedule_alone(wide):
         assert np.array_equal(a.E, b.E)
     one = sols['unset'][0]._engine
     assert nat.load().mmx_plan_chunk_ends(one.plan.handle, one.chi_kind) == 1
+
+
+@pytest.mark.parametrize('shape,components,launches', [((300,), 1, 'loop'), ((300,), 3, 'loop'), ((44, 60), 1, 'loop'),
+                                                       ((18, 20, 22), 3, 'loop'), ((44, 60), 1, 'passes'), ((300,), 1, 'passes')])
+@pytest.mark.parametrize('dtype', [np.complex64, np.complex128])
+def test_a_status_keeps_the_field(shape, components, launches, dtype):
+    """An update after one of norm 0 ends a right-hand side with MMX_STATUS_ZERODIV: its field is that before the update,
+    also when the last decision before had accepted one."""
+    from macromax_b200 import _native as nat, autotune
+    sol = _solution(_problem(shape, components, 'scalar'), dtype)
+    eng = sol._engine
+    autotune.set_variant(eng, _variants()[launches])
+    sol.solve(None, rtol=0, maxiter=4)
+    field = sol.E
+    st = eng.read_state()
+    assert st['accepted'][0] == 1
+    st['prev_norm'], st['active'], st['maxiter'] = 0.0, 1, np.inf
+    eng.write_state(st)
+    eng.iterate(3)
+    after = eng.read_state()
+    assert (after['status'][0], after['active'][0], after['iteration'][0]) == (nat.MMX_STATUS_ZERODIV, 0, 5)
+    assert after['cur'][0] == st['cur'][0]
+    assert np.array_equal(sol.E, field)
