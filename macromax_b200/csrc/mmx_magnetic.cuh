@@ -97,9 +97,10 @@ __global__ void __launch_bounds__(256) k_project_ft(const cpx<R>* F, cpx<R>* out
         const double inv = 1.0 / (k[0] * k[0] + k[1] * k[1] + k[2] * k[2]);
         cpx<R> proj = mkc<R>((R)0, (R)0);
 #pragma unroll
-        for (int c = 0; c < 3; ++c) proj += (R)k[c] * f[c];
+        for (int c = 0; c < 3; ++c)
+          if (c <= last) proj += (R)k[c] * f[c];  // (0 times an infinity is not 0)
 #pragma unroll
-        for (int c = 0; c < 3; ++c) pl[c] = (R)(k[c] * inv) * proj;
+        for (int c = 0; c < 3; ++c) pl[c] = c <= last ? (R)(k[c] * inv) * proj : mkc<R>((R)0, (R)0);
       }
 #pragma unroll
       for (int c = 0; c < 3; ++c) out[c * N + v] = transversal ? f[c] - pl[c] : pl[c];

@@ -1,0 +1,42 @@
+"""
+The projections of a 3-component spectrum in one kernel (mmx_project_ft), where the tensor expressions for other shapes and
+tracked tensors say what they give: components without an axis that are not finite.
+"""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+def _backend(shape, dtype):
+    from macromax_b200 import Grid
+    from macromax_b200.backend import BackEndB200
+    be = BackEndB200(3, Grid(shape=shape, step=125e-9), dtype)
+    rng = np.random.default_rng(2)
+    F = be.astype((rng.standard_normal((3, 1, *shape)) + 1j * rng.standard_normal((3, 1, *shape))).astype(dtype))
+    return be, F
+
+
+def _expressions(be, F, transversal):
+    """The same by tensor expressions."""
+    f = F.clone().requires_grad_(True)
+    out = be.transversal_projection_ft(f) if transversal else be.longitudinal_projection_ft(f)
+    assert out.requires_grad
+    return out.detach()
+
+
+@pytest.mark.parametrize('shape', [(7,), (130,), (13, 40), (64, 65)])
+@pytest.mark.parametrize('dtype', [np.complex64, np.complex128])
+@pytest.mark.parametrize('transversal', [False, True])
+def test_components_without_an_axis_stay_apart(shape, dtype, transversal):
+    be, F = _backend(shape, dtype)
+    last = (-1,) * len(shape)
+    F[(2, 0, *last)] = complex(np.inf, 0)
+    F[(2, 0, *(n // 2 for n in shape))] = complex(np.nan, np.nan)
+    out = be.transversal_projection_ft(F) if transversal else be.longitudinal_projection_ft(F)
+    got, ref = out.cpu().numpy(), _expressions(be, F, transversal).cpu().numpy()
+    nd = len(shape)
+    assert np.all(np.isfinite(got[:nd]))
+    tol = 4 * np.finfo(dtype).eps  # a few roundings per sample
+    assert np.linalg.norm(got[:nd] - ref[:nd]) <= tol * np.linalg.norm(F[:nd].cpu().numpy())
+    assert np.array_equal(got[nd:], ref[nd:], equal_nan=True)
