@@ -293,11 +293,13 @@ class BackEndB200:
         return self._k2
 
     def _project(self, F, transversal: bool):
-        """The projection of a 3-component field of this grid by mmx_project_ft; None for other shapes and for tensors
-        whose derivatives or batching torch tracks."""
-        if tuple(F.shape) != (3, 1, *(int(n) for n in self._grid.shape)) or F.requires_grad or \
-                torch._C._functorch.is_functorch_wrapped_tensor(F) or \
-                torch.autograd.forward_ad.unpack_dual(F).tangent is not None:
+        """The projection of a 3-component field of this grid by mmx_project_ft; None for other shapes, for tensors
+        whose derivatives or batching torch tracks, and while it records or intercepts operations (a launch of ours would
+        be missing there)."""
+        if tuple(F.shape) != (3, 1, *(int(n) for n in self._grid.shape)) or type(F) is not torch.Tensor or \
+                F.requires_grad or torch._C._functorch.is_functorch_wrapped_tensor(F) or \
+                torch.autograd.forward_ad.unpack_dual(F).tangent is not None or \
+                torch.jit.is_tracing() or torch.utils._python_dispatch._get_current_dispatch_mode() is not None:
             return None
         x = F.resolve_conj().resolve_neg().contiguous()
         out = torch.empty_like(x)

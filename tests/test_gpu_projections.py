@@ -1,6 +1,6 @@
 """
 The projections of a 3-component spectrum in one kernel (mmx_project_ft), where the tensor expressions for other shapes and
-tracked tensors say what they give: components without an axis that are not finite.
+tracked tensors say what they give: components without an axis that are not finite, and functions that torch records.
 """
 import numpy as np
 import pytest
@@ -40,3 +40,27 @@ def test_components_without_an_axis_stay_apart(shape, dtype, transversal):
     tol = 4 * np.finfo(dtype).eps  # a few roundings per sample
     assert np.linalg.norm(got[:nd] - ref[:nd]) <= tol * np.linalg.norm(F[:nd].cpu().numpy())
     assert np.array_equal(got[nd:], ref[nd:], equal_nan=True)
+
+
+@pytest.mark.parametrize('transversal', [False, True])
+def test_recorded_projections(transversal):
+    """torch.jit.trace, make_fx and a dispatch mode see the operations, and what they recorded serves other tensors."""
+    import torch
+    from torch.fx.experimental.proxy_tensor import make_fx
+    from torch.utils._python_dispatch import TorchDispatchMode
+    be, F = _backend((12, 10, 9), np.complex64)
+    project = be.transversal_projection_ft if transversal else be.longitudinal_projection_ft
+    other = torch.flip(F, (2, 3, 4)) * 0.5j
+    ref = _expressions(be, other, transversal)
+    seen = []
+
+    class Watch(TorchDispatchMode):
+        def __torch_dispatch__(self, func, types, args=(), kwargs=None):
+            seen.append(func)
+            return func(*args, **(kwargs or {}))
+
+    with Watch():
+        watched = project(other)
+    assert any('mul' in str(f) for f in seen)
+    for out in (watched, torch.jit.trace(project, (F,), check_trace=False)(other), make_fx(lambda x: project(x))(F)(other)):
+        assert torch.equal(out, ref)
