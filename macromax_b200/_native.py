@@ -144,8 +144,8 @@ def check(rc: int):
 
 def check_stalled(states):
     """Raise when a launch whose blocks wait for one another gave up (MMX_STATUS_STALLED): its fields are not valid."""
-    status = states['status']
-    if (int(status) if status.ndim == 0 else int(np.bitwise_or.reduce(status))) & MMX_STATUS_STALLED:
+    status = states['status']  # of one state or of an array of them
+    if (status.item() if status.size == 1 else int(np.bitwise_or.reduce(status))) & MMX_STATUS_STALLED:
         raise NativeError('the blocks of an iteration launch did not run together; set another variant '
                           '(MMX_VARIANT_PASSES) for this plan')
 

@@ -103,7 +103,7 @@ template <class R> LoopCfg loop_config(int ndim, const int64_t* shape, int C, in
     const int64_t most = std::max<int64_t>((int64_t)B * c.tiles[2], std::max<int64_t>((int64_t)B * c.tiles[0],
                                                                                     (int64_t)B * C * c.tiles[1]));
     if (most > 1 << 30) return c;
-    c.grid = (int)std::min<int64_t>(ctas, most);
+    c.grid = (int)std::min<int64_t>(std::min(ctas, (int)kLeaveGaveUp - 1), most);
     c.kept = (int)(((int64_t)B * c.tiles[2] + c.grid - 1) / c.grid);
     size_t work = 2 * (size_t)C * shape[0] * P0 * word;
     work = std::max(work, 2 * (size_t)C * c.PR * last * word);

@@ -267,9 +267,7 @@ __global__ void __launch_bounds__(kLoopThreads, sizeof(R) == 4 ? 2 : 1) k_loop(c
     if (tid == 0) {
       const LeaveResult r = leave_launch(gridDim.x, gave_up, [&](int word, unsigned v) {
         __threadfence();
-        const unsigned was = atomicAdd(a.counter + word, v);
-        __threadfence();
-        return was;
+        return atomicAdd(a.counter + word, v);
       });
       if (r.last)
         for (int w = 0; w < LEAVE_WORDS; ++w) a.counter[w] = 0u;

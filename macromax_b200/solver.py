@@ -324,7 +324,6 @@ class Solution:
     def _check_status(self, st):
         if int(st['status']) == nat.MMX_STATUS_ZERODIV:
             raise ZeroDivisionError('float division by zero (update norm after a zero update norm)')
-        nat.check_stalled(st)
 
     # -- iteration --------------------------------------------------------------------------------------------------
     def __iter__(self):
@@ -340,7 +339,9 @@ class Solution:
         self._engine.write_state(st)
         while True:
             self._engine.iterate(1)
-            st = self._engine.read_state()[0]
+            st = self._engine.read_state()
+            nat.check_stalled(st)
+            st = st[0]
             self._snapshot = (self._engine.state_key(), st)
             self._check_status(st)
             yield self
