@@ -269,16 +269,14 @@ __global__ void __launch_bounds__(256, GenBounds<R>::min_blocks) k_gen_strided(c
 // ---------------------------------------------------------------------------------------------------------------
 template <class R, int C, class Rad, class Sync>
 __device__ __forceinline__ void green_tile(const GenAxis& g, int lP, int ndim, unsigned inner, int64_t N, unsigned p,
-                                           cpx<R>* T0, double k1, double k2, double ar, double ai, cpx<R> h, double inv_total,
-                                           const gtw<R>* tw,
-                                           const double* sk0, cpx<R>* sm, int threads, Sync sync) {
+                                           cpx<R>* T0, double k1, double k2, GenGreen<R> green, cpx<R> h,
+                                           const gtw<R>* tw, const double* sk0, cpx<R>* sm, int threads, Sync sync) {
   const int n = g.n, P = 1 << lP, nst = g.nst;
   const size_t words = ((size_t)C * n) << lP;
   const int pl = threadIdx.x & (P - 1), slot = threadIdx.x >> lP, nslots = threads >> lP;
   const bool valid = p < inner;  // axis 0 has outer == 1: a pencil is its inner index
   cpx<R>* gp = T0 + p;
   const double kt2 = k1 * k1 + k2 * k2;
-  const GenGreen<R> green(ar, ai, inv_total);
   auto component = [&](int& i, int T) {  // i in [0, C T) -> component, i mod T
     int c = 0;
     if constexpr (C == 3) {
@@ -409,8 +407,8 @@ __global__ void __launch_bounds__(256, GenBounds<R>::min_blocks) k_gen_green(con
   const mmx_rhs_state* st = a.st + blockIdx.y;
   if (!st->active) return;
   green_tile<R, C, WideRadices>(a.g, a.lP, a.ndim, (unsigned)a.inner, a.N, p, a.T + (int64_t)blockIdx.y * C * a.N, k1, k2,
-                   st->alpha_re, st->alpha_im, gen_longitudinal<R>(st->alpha_re, st->alpha_im, a.inv_total_d), a.inv_total_d,
-                   tw, sk0, sm, blockDim.x, BlockSync());
+                   GenGreen<R>(st->alpha_re, st->alpha_im, a.inv_total_d),
+                   gen_longitudinal<R>(st->alpha_re, st->alpha_im, a.inv_total_d), tw, sk0, sm, blockDim.x, BlockSync());
 }
 
 // ---------------------------------------------------------------------------------------------------------------

@@ -46,16 +46,12 @@ enum : int { LOOP_EPI = 1, LOOP_PRO = 2 };
 // What the passes need of a right-hand side's state
 template <class R> struct LoopCoef {
   ChiCoef<R> cc;
-  double ar, ai;
+  GenGreen<R> green;
   cpx<R> h;
 };
 template <class R> __device__ __forceinline__ LoopCoef<R> loop_coef(const mmx_rhs_state* st, double inv_total) {
-  LoopCoef<R> c;
-  c.cc = chi_coef<R>(st);
-  c.ar = st->alpha_re;
-  c.ai = st->alpha_im;
-  c.h = gen_longitudinal<R>(c.ar, c.ai, inv_total);
-  return c;
+  const double ar = st->alpha_re, ai = st->alpha_im;
+  return LoopCoef<R>{chi_coef<R>(st), GenGreen<R>(ar, ai, inv_total), gen_longitudinal<R>(ar, ai, inv_total)};
 }
 
 // chi(alpha) v + (cc.s) s' of one sample from a kept tile (words of one component: `words`)
@@ -381,8 +377,8 @@ __global__ void __launch_bounds__(kLoopThreads, sizeof(R) == 4 ? 2 : 1) k_loop(c
         }
       }
       const LoopCoef<R>& q = coef[cur * B + b];
-      green_tile<R, C, SmallRadices>(a.g[0], a.lP0, ndim, inner0, N, p, a.T + (int64_t)b * C * N, k1, k2, q.ar, q.ai, q.h,
-                                     a.inv_total_d, tw(0), kt(0), sm, kLoopWorkers, sync);
+      green_tile<R, C, SmallRadices>(a.g[0], a.lP0, ndim, inner0, N, p, a.T + (int64_t)b * C * N, k1, k2, q.green, q.h,
+                                     tw(0), kt(0), sm, kLoopWorkers, sync);
       sync();
     }
   };
