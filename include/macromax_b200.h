@@ -125,7 +125,9 @@ int mmx_iterate(mmx_plan* plan, void* E0, void* E1, const void* chi, int chi_kin
  * mmx_iterate for `niter` iterations as one CUDA graph launch: the pass kernels are captured once per (plan,
  * buffers, niter) and replayed, which removes the per-kernel launch gaps that dominate small grids.  Same
  * semantics as mmx_iterate.  The captured graph is released with the plan.  Where a chunk runs in one launch
- * (mmx_plan_chunk_ends) there is no graph, and the launch is cooperative: its blocks wait for one another.
+ * (mmx_plan_chunk_ends) there is no graph, and the launch is cooperative: its blocks wait for one another, with a limit
+ * (MMX_STATUS_STALLED).  A launch that is refused because the context cannot hold its blocks at once runs in passes instead,
+ * and so do the plan's later ones.
  */
 int mmx_iterate_graph(mmx_plan* plan, void* E0, void* E1, const void* chi, int chi_kind, const void* src,
                       mmx_rhs_state* state, int niter, void* stream);
@@ -152,7 +154,9 @@ int mmx_iterate_graph_continue(mmx_plan* plan, void* E0, void* E1, const void* c
 /*
  * `niter` iterations of n independent problems (plans of possibly different grid shapes, e.g. an uneven batch of
  * 128^2, 256^2 and 384^2 grids) packed into ONE captured CUDA graph whose branches run concurrently.  Arrays of
- * length n give each plan's buffers as in mmx_iterate.  The reference solves such problems one after another.
+ * length n give each plan's buffers as in mmx_iterate.  Up to four plans whose chunks run in one launch
+ * (mmx_plan_chunk_ends) are launched after the graph, one after another, instead.  The reference solves such problems one
+ * after another.
  */
 int mmx_iterate_multi(int n, mmx_plan* const* plans, void* const* E0, void* const* E1, const void* const* chi,
                       const int* chi_kind, const void* const* src, mmx_rhs_state* const* state, int niter,

@@ -193,7 +193,9 @@ class UnevenBatch:
     """
     Several batches on grids of different sizes (e.g. 64 x 128^2, 32 x 256^2 and 8 x 384^2 sources) iterated by
     ONE captured CUDA graph per chunk of iterations (``mmx_iterate_multi``): each member's pass kernels form an
-    independent branch of the graph, so the small grids run concurrently instead of one after another.
+    independent branch of the graph, so the small grids run concurrently instead of one after another.  Members whose
+    chunks run in one launch (``mmx_plan_chunk_ends``) follow the graph one after another while there are at most four
+    of them; with more, all members are branches.
     """
 
     def __init__(self, members):

@@ -984,15 +984,17 @@ bool epro_runs(const mmx_plan* p, int chi_kind, int niter) {
 
 // The configuration under which a chunk of iterations runs in one launch, or null.  It does in the default variant where
 // the CTAs can keep the rows of the grid in shared memory (loop_config; up to about 900 000 scalar complex64 samples),
-// except on complex64 grids whose passes are all specialised for their length: those keep the rounding that their other
-// variants and their branch of an uneven batch have, and gain least.  us per iteration, one launch against passes:
+// except on complex64 grids whose passes are all specialised for their length: there a solve, its replay in a graph and its
+// branch of an uneven batch of any size give the same bits, and 512^2 and 64^3 gain little or nothing (64^2 and 256^2 would
+// gain a third; MMX_VARIANT_LOOP takes the one launch).  us per iteration, one launch against passes:
 // complex64 300 x 420 14.3 / 30.0, 8 sources on 200 x 180 19.0 / 29.6, 48 x 42 x 44 18.5 / 30.6 (vector: 23.5 / 33.5);
 // specialised: 64^2 9.3 / 13.1, 256^2 11.9 / 18.0, 512^2 22.4 / 24.0, 64^3 20.0 / 18.8; complex128 64^2 8.7 / 20.8, 256^2
 // 11.7 / 32.9, 512^2 23.1 / 29.6, 64^3 27.0 / 34.8; 1000 samples in 1D 6.2 / 20.0 (complex128 6.6 / 24.2).
-// Vector fields on 1D grids keep the passes too: a field along the only axis has a local Green function, its solve is often at
-// rounding level after 15 to 35 iterations, and from there on rounding alone says which updates the guard rejects.  Each
-// rejection raises alpha for good, so the results of the next solve of the same object would be others.
-// MMX_VARIANT_LOOP takes the one launch.
+// Vector fields on 1D grids keep the passes too: a field along the only axis has a local Green function, its solve is
+// often at rounding level after 15 to 35 iterations, and from there on rounding alone says which updates the guard rejects.
+// Each rejection raises alpha for good, so the results of the next solve of the same object would be others.
+// MMX_VARIANT_LOOP takes the one launch (300 samples 6.7 against 17.4 us, 800 samples 10.3 / 24.7; complex128 6.9 / 20.9
+// and 11.2 / 30.9).
 LoopCfg* loop_runs(mmx_plan* p, int chi_kind) {
   if (p->force_generic || p->no_reg || p->pipe || p->plane || p->epro || p->tma || p->runtime_radix || p->passes_only ||
       p->l2_persist)
@@ -1585,8 +1587,10 @@ int iterate_multi(int n, mmx_plan* const* plans, void* const* E0, void* const* E
     key.ints.push_back(chi_kind[i]);
   }
   // Chunks in one launch need no graph; their CTAs wait for one another, so they run one after another on the stream and
-  // not as branches.  Up to kLoopsInTurn members do so (the fields of a member are those of its own solve); with more, the
-  // branches of passes that run side by side are sooner done.
+  // not as branches.  Up to kLoopsInTurn members do so: a member's field then has the bits of its own solve.  That costs
+  // time from two or three members on, as branches of passes run side by side (us per iteration of 2 / 4 / 6 members of two
+  // sources, in turn and as branches: 60^2 22, 43, 64 and 22, 23, 25; 300^2 32, 63, 94 and 35, 40, 44; 40 x 36 x 44 41,
+  // 82, 122 and 32, 37, 45; 100 x 90 x 42 131, 261, 392 and 55, 80, 114); with more than four it would cost too much.
   constexpr int kLoopsInTurn = 4;
   std::vector<int> loops, rest;
   for (int i = 0; i < n; ++i) (loop_runs(plans[i], chi_kind[i]) ? loops : rest).push_back(i);

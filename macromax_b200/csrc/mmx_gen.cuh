@@ -7,9 +7,11 @@
 // run-time value: a stage is a switch over the radix around a fully unrolled butterfly, and the only divisions left,
 // of a butterfly's index by the stage's span and of a flat index by the butterflies per pencil, are multiplications by
 // a reciprocal that the host computes.  Stages between two shared-memory buffers need one barrier each.  What bounds
-// the passes is the traffic between L2 and the SMs; the runtime-radix passes of mmx_kernels.cuh (staged through shared
-// memory at both ends, out-of-line stages at a 64-register budget, integer divisions per element, twiddles from
-// global memory and O(r^2) butterflies for 7, 11 and 13) took five to ten times as long.
+// the passes is the issue of instructions (44-66% of the slots at 100 x 126 x 90, a third of them for addresses and indices;
+// mmx_len.cuh is these passes with the length known to the compiler); the runtime-radix passes of mmx_kernels.cuh
+// (staged through shared memory at both ends, out-of-line stages at a 64-register budget, integer divisions per element,
+// twiddles from global memory and O(r^2) butterflies for 7, 11 and 13) take three to four times as long (520 us per
+// iteration of that grid against 145).
 //
 // Strided tiles: P = 2^lP consecutive pencils, shared memory [component][sample][pencil]; a warp's accesses are whole
 // rows.  Contiguous tiles: P rows of every component, shared memory [row][sample] with a skew of one word per 128 bytes.
@@ -62,7 +64,7 @@ template <class R> using gtw = typename GenTw<R>::type;
 __device__ __forceinline__ unsigned gen_div(unsigned x, unsigned m) { return __umulhi(x, m); }
 
 // Radix policies: f(integral_constant<radix>) for the stage's radix.
-struct WideRadices {  // 2 .. 16: few stages, for passes that are bound by traffic
+struct WideRadices {  // 2 .. 16: few stages, so few exchanges and addresses, for passes of many tiles
   template <class F> static __device__ __forceinline__ void run(int r, F&& f) {
     switch (r) {
       case 2: f(std::integral_constant<int, 2>{}); break;
@@ -265,7 +267,8 @@ __global__ void __launch_bounds__(256, GenBounds<R>::min_blocks) k_gen_strided(c
 
 // ---------------------------------------------------------------------------------------------------------------
 // Axis 0: forward FFT, Green multiply, inverse FFT, in place, of the tile of pencils from tile << lP of one right-hand
-// side (T0: its first component).  h: i alpha_i / (alpha N), the longitudinal factor; sm: two buffers of C P n words; sk0: k of axis 0; k1, k2: of this thread's pencil.
+// side (T0: its first component).  h: i alpha_i / (alpha N), the longitudinal factor; sm: two buffers of C P n words; sk0: k
+// of axis 0; k1, k2: of this thread's pencil.
 // ---------------------------------------------------------------------------------------------------------------
 template <class R, int C, class Rad, class Sync>
 __device__ __forceinline__ void green_tile(const GenAxis& g, int lP, int ndim, unsigned inner, int64_t N, unsigned p,

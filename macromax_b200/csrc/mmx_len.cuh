@@ -1,6 +1,6 @@
 // The passes of mmx_gen.cuh compiled for one length: two stages of radix R0 and R1, N = R0 R1.
 //
-// The any-length passes are bound by the instructions they issue (55-66 % of the issue slots, a third of the instructions
+// The any-length passes are bound by the instructions they issue (44-66 % of the issue slots, a third of the instructions
 // for addresses and indices).  With the length, the tile and the block size known to the compiler the addresses become
 // immediate offsets, the loops unroll and the rows need no skew against bank conflicts: after the first stage a row is
 // kept in groups of R0 words at an odd pitch, which the second stage reads at that pitch.  The arithmetic is that of the

@@ -9,9 +9,10 @@
 //   in 3D the middle axis forward before and inverse after axis 0
 //
 // What bounds it is latency: a thread's instructions from one barrier to the next, and the trips to L2.  So the stages
-// have radices up to 10 (a radix-16 butterfly is one thread's work for a thousand cycles), and whatever a CTA meets again stays in shared memory: the fields, chi and
-// sources of its rows (loaded once, the fields written back at the end), the twiddles, the k tables, the states of the
-// right-hand sides and the coefficients that follow from them.  Only the work buffer crosses L2.
+// have radices up to 10 (a radix-16 butterfly is one thread's work for a thousand cycles), and whatever a CTA meets again
+// stays in shared memory: the fields, chi and sources of its rows (loaded once, the fields written back at the end), the
+// twiddles, the k tables, the states of the right-hand sides and the coefficients that follow from them.  Only the work
+// buffer crosses L2.
 //
 // The contiguous-axis tile goes on from E' to the next input chi E' + s'.  That is speculative, as in the fused epilogue
 // of mmx_epro.cuh: the divergence guard needs the norms of all tiles.  An extra warp of every CTA reduces them (each CTA

@@ -211,7 +211,8 @@ class MixedUnevenSolution:
     The mixed-precision solve for several batches on grids of different sizes (e.g. 64 x 128^2, 32 x 256^2 and
     8 x 384^2 sources of one material class): each member keeps its own FP64 iterate, defect and complex64 inner
     iteration (a MixedSolution), and in every outer step the inner solves of all members run together, one captured
-    CUDA graph per chunk of iterations with each member's passes as an independent branch (UnevenBatch).
+    CUDA graph per chunk of iterations with each member's passes as an independent branch, or up to four members whose
+    chunks run in one launch after it (UnevenBatch).
     """
 
     def __init__(self, members):
